@@ -1,0 +1,123 @@
+// leo_slice.cu -- launches of the bit-sliced Leopard GF(2^8) transforms
+// (slice_fft.cuh).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdlib>
+
+#include "codec.hpp"
+#include "launch_cfg.hpp"
+#include "leo_slice.hpp"
+#include "slice_fft.cuh"
+
+namespace rsgpu {
+
+#define RS_CUDA(expr)                              \
+  do {                                             \
+    cudaError_t e_ = (expr);                       \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
+  } while (0)
+
+namespace {
+
+constexpr int kSliceMaxThreads = 1024;  // 64 registers
+
+template <int WT, bool VERIFY>
+__global__ void __launch_bounds__(kSliceMaxThreads, 1) k_slice_encode(SliceArgs a) {
+  extern __shared__ __align__(16) uint4 slice_smem[];
+  constexpr uint64_t tile_bytes = 32 * WT;
+  const uint32_t tiles_per_job = uint32_t((a.len + tile_bytes - 1) / tile_bytes);
+  const uint32_t total = tiles_per_job * a.n_jobs;
+#pragma unroll 1
+  for (uint32_t x = blockIdx.x; x < total; x += gridDim.x) {
+    const uint32_t job = x / tiles_per_job;
+    const uint64_t tile = uint64_t(x - job * tiles_per_job) * tile_bytes;
+    const LeoJob jd = a.jobs[job];
+    const uint32_t bad = slice_encode_tile<WT, VERIFY>(uint32_t(__cvta_generic_to_shared(slice_smem)), a, a.ptrs + jd.ptr_off, tile, a.len);
+    if (VERIFY && __any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(a.flags + jd.flag_idx, 1u);
+    __syncthreads();  // rows are free for the next tile
+  }
+}
+
+template <int WT>
+__global__ void __launch_bounds__(kSliceMaxThreads, 1) k_slice_decode(SliceArgs a) {
+  extern __shared__ __align__(16) uint4 slice_smem[];
+  __shared__ __align__(8) uint8_t need_bits[8];
+  uint64_t *lane_ptrs = reinterpret_cast<uint64_t *>(slice_smem + size_t(a.n) * 2 * WT);
+  const LaneInfo info{lane_ptrs, reinterpret_cast<uint8_t *>(lane_ptrs + a.n)};
+  constexpr uint64_t tile_bytes = 32 * WT;
+  const uint32_t tiles_per_job = uint32_t((a.len + tile_bytes - 1) / tile_bytes);
+  const uint32_t total = tiles_per_job * a.n_jobs;
+  uint32_t cur = ~0u;
+#pragma unroll 1
+  for (uint32_t x = blockIdx.x; x < total; x += gridDim.x) {
+    const uint32_t job = x / tiles_per_job;
+    if (job != cur) {  // CTA-uniform; the rows and info are free (barrier below)
+      cur = job;
+      slice_lane_info(a, a.jobs[job], info, need_bits);
+      __syncthreads();
+    }
+    slice_decode_tile<WT>(uint32_t(__cvta_generic_to_shared(slice_smem)), a, info, need_bits, a.jobs[job].input_count,
+                          uint64_t(x - job * tiles_per_job) * tile_bytes, a.len);
+    __syncthreads();
+  }
+}
+
+// Rows of a tile: decode n lanes; encode the accumulator and, with more than
+// one data group, the scratch.
+uint32_t slice_rows(int op, uint32_t k, uint32_t m, uint32_t n) {
+  return op == RSGPU_OP_RECONSTRUCT ? n : (k > m ? 2 * m : m);
+}
+
+using SliceKernel = void (*)(SliceArgs);
+SliceKernel slice_kernel(int op, uint32_t wt) {
+  if (op == RSGPU_OP_RECONSTRUCT) return wt == 32 ? k_slice_decode<32> : k_slice_decode<28>;
+  if (op == RSGPU_OP_VERIFY) return wt == 32 ? k_slice_encode<32, true> : k_slice_encode<28, true>;
+  return wt == 32 ? k_slice_encode<32, false> : k_slice_encode<28, false>;
+}
+
+}  // namespace
+
+bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t columns) {
+  if (op == RSGPU_OP_RECONSTRUCT) return n > 8 || columns >= (512 << 10);
+  if (m > 16) return true;
+  return k <= 4 * m && (m == 16 || columns >= (2 << 20));
+}
+
+int slice_configure(int op, SliceArgs &a, SliceShape &sh) {
+  constexpr size_t kLimit = 227 * 1024 - 256;  // a CTA's shared memory less the static part
+  a.rows = slice_rows(op, a.k, a.m, a.n);
+  const size_t info = op == RSGPU_OP_RECONSTRUCT ? size_t(a.n) * LaneInfo::kBytes : 0;
+  const uint32_t lanes = op == RSGPU_OP_RECONSTRUCT ? a.n : a.m;
+  const uint32_t items = std::max(1u, lanes / 4);  // radix-4 groups of a pass: one per warp
+  a.wt = 32;
+  // 28 threads a row when 256 rows would not fit at 32, and when it lets a
+  // second CTA share the SM (128 rows).
+  if (size_t(a.rows) * 32 * a.wt + info > kLimit || (a.rows == 128 && !info)) a.wt = 28;
+  sh.smem = size_t(a.rows) * 32 * a.wt + info;
+  const uint32_t ctas = std::max<uint32_t>(1, uint32_t(227 * 1024 / (sh.smem + 1280)));
+  uint32_t warps = 1;
+  while (warps * 2 <= items && warps * 2 * ctas <= 32 + 16) warps *= 2;
+  sh.threads = int(32 * std::min(warps, 32u));
+  const void *fn = reinterpret_cast<const void *>(slice_kernel(op, a.wt));
+  RS_CUDA(ensure_smem_limit(fn, sh.smem));
+  int per_sm = 0;
+  RS_CUDA(blocks_per_sm(fn, sh.threads, sh.smem, &per_sm));
+  const uint64_t tile = uint64_t(32) * a.wt;
+  const uint64_t tiles = ((a.len + tile - 1) / tile) * std::max<uint32_t>(a.n_jobs, 1);
+  sh.grid = int(std::min<uint64_t>(tiles, uint64_t(std::max(per_sm, 1)) * device_sm_count()));
+  return RSGPU_OK;
+}
+
+int slice_launch(int op, const SliceArgs &a, const SliceShape &sh, cudaStream_t s) {
+  slice_kernel(op, a.wt)<<<sh.grid, sh.threads, sh.smem, s>>>(a);
+  launch_counter_add(1);
+  return cuda_status(cudaGetLastError());
+}
+
+// Tower coordinates of the element of each log value (exp: Cantor coordinates).
+void slice_elements(const uint16_t *exp, uint32_t order, uint16_t *out) {
+  for (uint32_t i = 0; i < order; ++i) out[i] = uint16_t(cantor_to_tower<8>(exp[i]));
+}
+
+}  // namespace rsgpu

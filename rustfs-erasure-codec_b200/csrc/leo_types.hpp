@@ -44,4 +44,17 @@ struct LeoArgs {
   uint32_t n_ienc, n_fenc, n_idec, n_fdec;
 };
 
+// Launch of the bit-sliced GF(2^8) transforms (slice_fft.cuh).
+struct SliceArgs {
+  const LeoJob *jobs;
+  const uint8_t *const *ptrs;
+  uint32_t *flags;
+  const uint16_t *elem;  // per log value: the element's tower coordinates
+  uint64_t len;          // bytes per shard (multiple of 64)
+  uint32_t n_jobs;
+  uint32_t k, p, m, n, mod;
+  uint32_t wt;  // threads per row: a tile is 32 * wt bytes of every shard
+  uint32_t rows;
+};
+
 }  // namespace rsgpu

@@ -35,6 +35,7 @@
 
 #include "codec.hpp"
 #include "leo_fft.cuh"
+#include "leo_slice.hpp"
 #include "leo_tile.cuh"
 #include "launch_cfg.hpp"
 #include "leopard.hpp"
@@ -149,6 +150,7 @@ struct LeoField {
   uint32_t *d_bank = nullptr;   // multiplier tables indexed by log value (half-warp layer kernels)
   uint32_t *d_kbank = nullptr;  // tables of the register-stage kernels (GF(2^8): 5+3 split; GF(2^16): 5+5+5+1)
   uint32_t *d_sktab = nullptr;  // d_kbank's entry of each skew entry: entry i holds the tables of log skew[i]
+  uint16_t *d_elem = nullptr;   // GF(2^8): tower coordinates of each log's element (slice_field.cuh)
   uint8_t *d_mul8 = nullptr;    // GF(2^8): products mul[a][b], 256 x 256 (device packing of dense maps)
   explicit LeoField(int b) : bits(b), host(b) {}
 };
@@ -211,6 +213,10 @@ static int leo_field(int bits, LeoField **out) {
         for (uint32_t b = 1; b < 256; ++b) mul[a * 256 + b] = uint8_t(t.exp[t.add_mod(t.log[a], t.log[b])]);
       RS_CUDA(cudaMalloc(&f->d_mul8, mul.size()));
       RS_CUDA(cudaMemcpy(f->d_mul8, mul.data(), mul.size(), cudaMemcpyHostToDevice));
+      std::vector<uint16_t> elem(t.order);
+      slice_elements(t.exp.data(), t.order, elem.data());
+      RS_CUDA(cudaMalloc(&f->d_elem, elem.size() * 2));
+      RS_CUDA(cudaMemcpy(f->d_elem, elem.data(), elem.size() * 2, cudaMemcpyHostToDevice));
     } else {
       // Per log value, 32 lanes x 4 words (layout of leo_fft.cuh): c * i,
       // c * (i << 5), c * (i << 10) for i = lane, and c * 2^15, each
@@ -476,8 +482,12 @@ struct LeopardState {
 struct LeoLaunch {
   Codec *codec = nullptr;
   bool decode = false, verify = false;
-  int engine = 1;  // 1: register-stage kernels, 0: half-warp layer kernels
+  // 2: bit-sliced GF(2^8) kernels, 1: register-stage kernels, 0: half-warp
+  // layer kernels.
+  int engine = 1;
   LeoArgs args{};
+  SliceArgs slice{};
+  SliceShape slice_shape;
   void *d_blob = nullptr;  // jobs | pointers | roles
   // One-shot launches allocate the blob on their stream and free it there
   // after the kernel; prepared launches own it until destroyed.
@@ -1008,6 +1018,28 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
   a.sktab = st.field->d_sktab;
   fill_stages(a);
   L.engine = leo_engine();
+  if (L.engine == 1 && st.field->bits == 8) {
+    // The bit-sliced kernels read shards 16 bytes at a time; other pointers
+    // stay on the register-stage kernels' 4-byte accesses.
+    uintptr_t low = 0;
+    for (size_t i = 0; i < n_stripes * total; ++i) low |= reinterpret_cast<uintptr_t>(shards[i]);
+    if ((low & 15) == 0 && slice_pays(op, a.k, a.m, a.n, uint64_t(len) * a.n_jobs)) {
+      L.engine = 2;
+      SliceArgs &sa = L.slice;
+      sa.jobs = a.jobs;
+      sa.ptrs = a.ptrs;
+      sa.flags = flags;
+      sa.elem = st.field->d_elem;
+      sa.len = len;
+      sa.n_jobs = a.n_jobs;
+      sa.k = a.k;
+      sa.p = a.p;
+      sa.m = a.m;
+      sa.n = a.n;
+      sa.mod = a.mod;
+      return slice_configure(op, sa, L.slice_shape);
+    }
+  }
   if (L.engine == 1) {
     const bool b16f = st.field->bits == 16;
     const size_t nj = jobs.size();
@@ -1071,6 +1103,9 @@ namespace {
 int leo_launch_kernel(const LeoLaunch &L, cudaStream_t s) {
   const bool b16 = L.codec->leo->field->bits == 16;
   const LeoArgs &a = L.args;
+  if (L.engine == 2)
+    return slice_launch(L.decode ? RSGPU_OP_RECONSTRUCT : L.verify ? RSGPU_OP_VERIFY : RSGPU_OP_ENCODE, L.slice,
+                        L.slice_shape, s);
   if (L.engine == 1) {
     const dim3 grid(L.grid), block(L.threads);
     const bool wide = L.threads != kFftThreads;
