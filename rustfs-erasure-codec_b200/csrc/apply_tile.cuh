@@ -90,6 +90,109 @@ __device__ __forceinline__ void st_stream(uint8_t *p, uint4 v) {
                : "memory");
 }
 
+// ------------------------------------------------------------------ shared lookups
+// Lookup tables of C inputs (C = 1, 3 or 5) for four packed outputs, one entry
+// of 32 per lane.  A shuffle reads a table of 32 entries, i.e. five bits of
+// data, so looking bytes up one by one (two lookups each) wastes two bits of
+// ten.  Here each byte's low five bits index its input's own table and the
+// high bits of several inputs, three each, are packed five to a lookup: five
+// inputs take 5 + 3 lookups a column instead of 10, three take 3 + 2.  The
+// packing is done on whole words (four columns at once), so the integer work
+// per lookup stays where it was.
+//   mixed index 0: bits 5-7 of input 0, bits 5-6 of input 1
+//   mixed index 1: bit 7 of input 1, bits 5-7 of input 2, bit 5 of input 3
+//   mixed index 2: bits 6-7 of input 3, bits 5-7 of input 4
+template <int C>
+struct Lut {
+  static constexpr int kMixed = (3 * C + 4) / 5;
+  uint32_t low[C], mix[kMixed];
+};
+
+// tab(i, w): word w of input i's packed table (layout of common.hpp; words
+// 16..63 are used: 16 + n holds c * (n << 4), 32 + n holds c * n).
+template <int C, class T>
+__device__ __forceinline__ void lut_load(Lut<C> &t, uint32_t lane, T tab) {
+#pragma unroll
+  for (int i = 0; i < C; ++i) t.low[i] = tab(i, 32 + lane);
+  const uint32_t l = lane;
+  if (C == 1) {
+    t.mix[0] = tab(0, 16 + 2 * (l & 7));  // repeated: the index's bits 3-4 do not matter
+    return;
+  }
+  t.mix[0] = tab(0, 16 + 2 * (l & 7)) ^ tab(1 % C, 16 + 2 * (l >> 3));
+  t.mix[1 % Lut<C>::kMixed] = tab(1 % C, 16 + 8 * (l & 1)) ^ tab(2 % C, 16 + 2 * ((l >> 1) & 7));
+  if (C == 5) {
+    t.mix[1 % Lut<C>::kMixed] ^= tab(3 % C, 16 + 2 * (l >> 4));
+    t.mix[2 % Lut<C>::kMixed] = tab(3 % C, 16 + 4 * (l & 3)) ^ tab(4 % C, 16 + 2 * (l >> 2));
+  }
+}
+
+// Mixed index words of one word of each input.
+template <int C>
+__device__ __forceinline__ void lut_index(const uint32_t *x, uint32_t *m) {
+  if (C == 1) {
+    m[0] = x[0] >> 5;
+    return;
+  }
+  m[0] = ((x[0] >> 5) & 0x07070707u) | ((x[1 % C] >> 2) & 0x18181818u);
+  uint32_t m1 = ((x[1 % C] >> 7) & 0x01010101u) | ((x[2 % C] >> 4) & 0x0E0E0E0Eu);
+  if (C == 5) {
+    m1 |= (x[3 % C] >> 1) & 0x10101010u;
+    m[2 % Lut<C>::kMixed] = ((x[3 % C] >> 6) & 0x03030303u) | ((x[4 % C] >> 3) & 0x1C1C1C1Cu);
+  }
+  m[1 % Lut<C>::kMixed] = m1;
+}
+
+// acc[0..3] ^= the products of one word (four columns) of each input.
+template <int C>
+__device__ __forceinline__ void lut_mac(const Lut<C> &t, const uint32_t *x, const uint32_t *m, uint32_t *acc) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) acc[b] ^= tshfl(t.low[i], x[i] >> (8 * b));
+#pragma unroll
+    for (int i = 0; i < Lut<C>::kMixed; ++i) acc[b] ^= tshfl(t.mix[i], m[i] >> (8 * b));
+  }
+}
+
+// The lookups of K inputs: fives, then a three, then singles.
+template <int K>
+struct LutSet {
+  static constexpr int kFive = K / 5, kThree = K % 5 >= 3 ? 1 : 0, kOne = K % 5 - 3 * kThree;
+  Lut<5> five[kFive ? kFive : 1];
+  Lut<3> three;
+  Lut<1> one[kOne ? kOne : 1];
+  // tbl: the packed table of four outputs over K inputs.
+  __device__ __forceinline__ void load(const uint32_t *tbl, uint32_t lane) {
+    auto at = [&](int j0) {
+      return [=](int i, uint32_t w) { return __ldg(tbl + (j0 + i) * kTableWords + w); };
+    };
+#pragma unroll
+    for (int q = 0; q < kFive; ++q) lut_load<5>(five[q], lane, at(5 * q));
+    if (kThree) lut_load<3>(three, lane, at(5 * kFive));
+#pragma unroll
+    for (int q = 0; q < kOne; ++q) lut_load<1>(one[q], lane, at(5 * kFive + 3 * kThree + q));
+  }
+  // acc[0..3] ^= the products of one word of every input.
+  __device__ __forceinline__ void mac(const uint32_t *x, uint32_t *acc) const {
+    uint32_t m[3];
+#pragma unroll
+    for (int q = 0; q < kFive; ++q) {
+      lut_index<5>(x + 5 * q, m);
+      lut_mac<5>(five[q], x + 5 * q, m, acc);
+    }
+    if (kThree) {
+      lut_index<3>(x + 5 * kFive, m);
+      lut_mac<3>(three, x + 5 * kFive, m, acc);
+    }
+#pragma unroll
+    for (int q = 0; q < kOne; ++q) {
+      lut_index<1>(x + 5 * kFive + 3 * kThree + q, m);
+      lut_mac<1>(one[q], x + 5 * kFive + 3 * kThree + q, m, acc);
+    }
+  }
+};
+
 // One tile = kApplyThreads threads x V 128-bit vectors of columns of job d,
 // starting at byte tile_base (< d.vec_len).  NG = number of 4-output groups
 // per pass over the inputs (outputs g*4 .. g*4+3).  MIX: 0 = every input uses

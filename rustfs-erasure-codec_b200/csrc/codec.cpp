@@ -446,11 +446,12 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
                        uint32_t *flags, cudaStream_t s, bool persistent, bool accumulate) {
   verify = vfy;
   max_tail = 0;
-  uint32_t max_out = 0;
+  uint32_t max_out = 0, uni_in = jobs.empty() ? 0 : jobs[0].n_in;
   int any_vec = 0;
   int tbl_stage = 0;
   for (auto &j : jobs) {
     tbl_stage |= j.tbl != jobs[0].tbl;
+    if (j.n_in != uni_in) uni_in = 0;
     bool aligned = true;
     const uint32_t n_ptr = uint32_t(j.n_in) + j.n_out * (j.verify_store ? 2u : 1u);
     for (uint32_t i = 0; i < n_ptr; ++i)
@@ -478,6 +479,7 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   args.len = len;
   args.n_jobs = uint32_t(jobs.size());
   args.max_out = max_out;
+  args.uni_in = uni_in;
   args.any_vec = any_vec;
   args.tbl_stage = tbl_stage;
   args.accumulate = accumulate ? 1 : 0;

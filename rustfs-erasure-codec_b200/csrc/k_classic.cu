@@ -263,6 +263,170 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a
   }
 }
 
+// ------------------------------------------------------------------ K1, tables in registers
+// The product for at most 4 outputs over K <= kRegInputs inputs, all lookup
+// tables of the K inputs in registers (8 per five inputs, see apply_tile.cuh),
+// loaded when the CTA meets another table, so the loop over columns is nothing
+// but data reads, shuffles and XORs.  What bounds it is the L1 data pipe: of
+// about 8 wavefronts per input word (128 bytes a warp) 6.4 are shuffles, 1 is
+// the data read.  The staged tile above needs 8 shuffles and re-reads two
+// tables per input and step, in 96 registers; this one fits 72, so three CTAs
+// share an SM and the shuffle latency is hidden (10+4 encode, 1 MiB x 512:
+// 4498 -> 5351 GB/s, 83% of the copy peak; the pipe is 81% busy).
+// A CTA takes a contiguous run of tiles: launches whose stripes carry
+// different tables then change tables once per stripe, not once per tile.
+// The producer warp, the mbarrier ring and its bounded waits are
+// k_apply_tma's; a stage is one tile of all K inputs (for verify also the <= 4
+// parity shards).
+constexpr int kRegInputs = 20;
+
+template <int K, bool VERIFY>
+struct RegShape {
+  static constexpr int kSlots = K + (VERIFY ? 4 : 0);
+  // Words a thread reads at a time: two (64-bit reads) while they fit the
+  // registers of three CTAs an SM.
+  static constexpr int kWords = K <= 10 ? 2 : 1;
+  // Bytes of every shard a tile: enough work between two barrier waits.
+  static constexpr uint32_t kTile = K <= 4 ? 8192 : K <= 7 ? 4096 : 2048;
+  static constexpr int kFit = int(74 * 1024 / (kSlots * kTile));
+  static constexpr int kStages = kFit < 2 ? 2 : kFit > 4 ? 4 : kFit;
+  static constexpr int kBlocks = kFit < 2 || K > 13 ? 2 : 3;
+  static constexpr size_t kSmem = size_t(kStages) * kSlots * kTile;
+};
+
+template <int K, bool VERIFY>
+__global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBlocks) k_apply_reg(ApplyArgs a) {
+  using Shape = RegShape<K, VERIFY>;
+  constexpr int S = Shape::kStages, W = Shape::kWords;
+  constexpr uint32_t kTile = Shape::kTile, kStageBytes = Shape::kSlots * kTile;
+  extern __shared__ __align__(128) uint8_t reg_smem[];
+  __shared__ __align__(8) uint64_t full[S], empty[S];
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t sbase = uint32_t(__cvta_generic_to_shared(reg_smem));
+  const uint32_t fbar = uint32_t(__cvta_generic_to_shared(full));
+  const uint32_t ebar = uint32_t(__cvta_generic_to_shared(empty));
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(fbar + 8 * s, 1);
+      mbar_init(ebar + 8 * s, kApplyThreads / 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const uint32_t tiles_per_job = uint32_t((a.len + kTile - 1) / kTile);
+  const uint64_t total = uint64_t(tiles_per_job) * a.n_jobs;
+  const uint32_t t0 = uint32_t(total * blockIdx.x / gridDim.x), t1 = uint32_t(total * (blockIdx.x + 1) / gridDim.x);
+  uint32_t job = t0 / tiles_per_job, tile = t0 - job * tiles_per_job;
+  uint32_t s = 0, ph = 0;  // ring position and its phase
+
+  if (tid >= kApplyThreads) {  // producer warp: one lane issues every copy
+    if (tid != kApplyThreads) return;
+    uint32_t issued = 0;
+    bool ok = true;
+    for (uint32_t t = t0; t < t1; ++t) {
+      const JobDesc d = a.jobs[job];
+      const uint64_t base = uint64_t(tile) * kTile;
+      if (base < d.vec_len) {
+        const uint32_t valid = uint32_t(d.vec_len - base < kTile ? d.vec_len - base : kTile);
+        const uint32_t rows = K + (VERIFY ? d.n_out : 0);
+        const uint8_t *const *ptr = a.ptrs + d.ptr_off;
+        if (!mbar_wait(ebar + 8 * s, ph ^ 1)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(fbar + 8 * s, rows * valid);
+        for (uint32_t b = 0; b < rows; ++b)
+          bulk_load(sbase + s * kStageBytes + b * kTile, ptr[b] + base, valid, fbar + 8 * s);
+        ++issued;
+        if (++s == S) s = 0, ph ^= 1;
+      }
+      if (++tile == tiles_per_job) tile = 0, ++job;
+    }
+    if (!ok) {
+      if (a.stall) atomicOr(a.stall, 1u);
+      // Wait (bounded) for the copies in flight before the CTA's shared
+      // memory goes away: the last min(S, issued) stages.
+      for (uint32_t k = 0; k < S && k < issued; ++k) {
+        if (s == 0) s = S, ph ^= 1;
+        --s;
+        mbar_wait(fbar + 8 * s, ph);
+      }
+    }
+    return;
+  }
+
+  LutSet<K> lut;
+  const uint32_t *cur = nullptr;
+  JobDesc d{};
+  uint8_t *dst[4];  // this job's outputs (verify: where verify_store puts them)
+  bool fresh = true;
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint64_t base = uint64_t(tile) * kTile;
+    if (fresh) {
+      fresh = false;
+      d = a.jobs[job];
+      const uint8_t *const *out = a.ptrs + d.ptr_off + K + (VERIFY ? d.n_out : 0);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        dst[r] = uint32_t(r) < d.n_out && (!VERIFY || d.verify_store) ? const_cast<uint8_t *>(out[r]) : nullptr;
+      if (d.tbl != cur) {
+        lut.load(d.tbl, lane);
+        cur = d.tbl;
+      }
+    }
+    if (base < d.vec_len) {
+      if (!mbar_wait(fbar + 8 * s, ph)) {
+        if (a.stall) atomicOr(a.stall, 1u);
+        return;
+      }
+      bool bad = false;
+#pragma unroll 1
+      for (uint32_t sub = 0; sub < kTile / (kApplyThreads * 4 * W); ++sub) {
+        if (base + sub * (kApplyThreads * 4 * W) >= d.vec_len) break;  // CTA-uniform
+        const uint32_t off = (sub * kApplyThreads + tid) * 4 * W;
+        const uint32_t slot = sbase + s * kStageBytes + off;
+        uint32_t x[W][K], acc[W][4];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          if (W == 2)
+            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x[0][j]), "=r"(x[W - 1][j]) : "r"(slot + j * kTile) : "memory");
+          else
+            x[0][j] = lds32(slot + j * kTile);
+        }
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          uint32_t o[4] = {0, 0, 0, 0};
+          lut.mac(x[w], o);
+          transpose4(o, acc[w]);
+        }
+        const uint64_t col = base + off;
+        if (col < d.vec_len) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            if (VERIFY && uint32_t(r) < d.n_out) {
+#pragma unroll
+              for (int w = 0; w < W; ++w) bad |= lds32(slot + (K + r) * kTile + 4 * w) != acc[w][r];
+            }
+            if (dst[r]) {
+              if (W == 2)
+                asm volatile("st.global.L1::no_allocate.v2.u32 [%0], {%1,%2};" ::"l"(dst[r] + col), "r"(acc[0][r]),
+                             "r"(acc[W - 1][r])
+                             : "memory");
+              else
+                asm volatile("st.global.L1::no_allocate.u32 [%0], %1;" ::"l"(dst[r] + col), "r"(acc[0][r]) : "memory");
+            }
+          }
+        }
+      }
+      if (VERIFY && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags + d.flag_idx, 1u);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ebar + 8 * s);
+      if (++s == S) s = 0, ph ^= 1;
+    }
+    if (++tile == tiles_per_job) tile = 0, ++job, fresh = true;
+  }
+}
+
 // Byte-granular path for the columns past each job's vec_len.  One thread per
 // byte column.
 template <bool VERIFY, bool ACC = false>
@@ -467,20 +631,50 @@ void launch_tma(const ApplyArgs &a, cudaStream_t s) {
   k_apply_tma<V, S, VERIFY><<<grid, kApplyThreads + 32, smem, s>>>(a);
 }
 
-// Tile variants the autotuner chooses from: (vectors per thread, inputs in
-// flight, lookup mix).
+template <int K, bool VERIFY>
+void launch_reg(const ApplyArgs &a, cudaStream_t s) {
+  using Shape = RegShape<K, VERIFY>;
+  static int grid_max = 0;
+  const void *fn = (const void *)k_apply_reg<K, VERIFY>;
+  ensure_smem_limit(fn, Shape::kSmem + 512);  // with the static part it may pass 48 KiB
+  if (!grid_max) grid_max = grid_for(fn, kApplyThreads + 32, Shape::kSmem);
+  const uint64_t tiles = ((a.len + Shape::kTile - 1) / Shape::kTile) * a.n_jobs;
+  const int grid = int(tiles < uint64_t(grid_max) ? tiles : grid_max);
+  k_apply_reg<K, VERIFY><<<grid, kApplyThreads + 32, Shape::kSmem, s>>>(a);
+}
 template <bool VERIFY>
-void launch_variant(const ApplyArgs &a, int variant, cudaStream_t s) {
-  if (a.max_out > 4) {
+void launch_reg_k(const ApplyArgs &a, cudaStream_t s) {
+  switch (a.uni_in) {
+#define RS_REG_CASE(K) \
+  case K: launch_reg<K, VERIFY>(a, s); break;
+    RS_REG_CASE(1) RS_REG_CASE(2) RS_REG_CASE(3) RS_REG_CASE(4) RS_REG_CASE(5) RS_REG_CASE(6) RS_REG_CASE(7)
+    RS_REG_CASE(8) RS_REG_CASE(9) RS_REG_CASE(10) RS_REG_CASE(11) RS_REG_CASE(12) RS_REG_CASE(13) RS_REG_CASE(14)
+    RS_REG_CASE(15) RS_REG_CASE(16) RS_REG_CASE(17) RS_REG_CASE(18) RS_REG_CASE(19) RS_REG_CASE(20)
+#undef RS_REG_CASE
+    default: break;
+  }
+}
+
+// More than 4 outputs: the register-path tile, 8 outputs a pass.  At most 4:
+// tables in registers up to kRegInputs inputs a job (beyond, they no longer
+// fit), the staged tile with tables read per step for wider jobs and for
+// launches whose jobs differ in width.  One B200, GB/s, staged tile / tables
+// in registers:
+//   encode 10+4   1 MiB x 512 4498 / 5351, 64 KiB x 256 3544 / 4374, 8 KiB x 1024 2890 / 3731
+//   encode 4+2    1 MiB x 512 4476 / 5345;  16+4 1 MiB x 256 4209 / 4807
+//   encode 8+4    4 KiB x 4096 2175 / 4278
+//   rebuild 16+4  1 MiB x 256 4109 / 4604;  6+3 256 KiB x 512 4102 / 4765
+//   verify 20+4   1 MiB x 128 4036 / 4231
+template <bool VERIFY>
+void launch_write_or_verify(const ApplyArgs &a, int variant, cudaStream_t s) {
+  if (a.max_out > 4)
     launch_vec<2, 1, 4, 1, VERIFY>(a, s);
-    return;
-  }
-  switch (variant) {
-    case 1: launch_vec<1, 2, 4, 0, VERIFY>(a, s); break;  // register path
-    case 2: launch_tma<2, 2, VERIFY>(a, s); break;
-    case 3: launch_tma<1, 4, VERIFY>(a, s); break;
-    default: launch_tma<2, 3, VERIFY>(a, s); break;  // 0: TMA-staged, 2 x 16 B per thread, 3 stages
-  }
+  else if (variant == 1)
+    launch_vec<1, 2, 4, 0, VERIFY>(a, s);
+  else if (variant == 0 && a.uni_in >= 1 && a.uni_in <= kRegInputs)
+    launch_reg_k<VERIFY>(a, s);
+  else
+    launch_tma<2, 3, VERIFY>(a, s);
 }
 
 }  // namespace
@@ -500,9 +694,9 @@ cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cud
     if (a.accumulate)
       launch_vec<1, 2, 4, 0, false, true>(a, s);
     else if (verify)
-      launch_variant<true>(a, apply_variant(), s);
+      launch_write_or_verify<true>(a, apply_variant(), s);
     else
-      launch_variant<false>(a, apply_variant(), s);
+      launch_write_or_verify<false>(a, apply_variant(), s);
     ++launches;
   }
   if (max_tail) {

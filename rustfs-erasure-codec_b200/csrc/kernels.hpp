@@ -15,15 +15,16 @@ struct ApplyArgs {
   uint64_t len;                 // bytes per shard (same for every job)
   uint32_t n_jobs;
   uint32_t max_out;             // largest n_out over the jobs
+  uint32_t uni_in;              // n_in of every job, 0 when they differ
   int any_vec;                  // some job has vec_len > 0
   int accumulate;               // outputs ^= products (incremental parity update)
   uint32_t *stall;              // device status word: a bounded wait of the TMA-staged tile ran out (may be null)
   int tbl_stage;                // jobs carry different tables: the TMA-staged tile copies them with the data
 };
 cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cudaStream_t s);
-// K1 tile for launches of at most 4 outputs: 0 (default) TMA-staged, 1 the
-// register-path tile, 2 / 3 other TMA ring shapes; RSGPU_APPLY_VARIANT picks
-// one for measurements.
+// K1 tile for launches of at most 4 outputs: 0 (default) tables in registers
+// where they fit, 1 the register-path tile, 2 the staged tile throughout;
+// RSGPU_APPLY_VARIANT picks one for measurements.
 int &apply_variant();
 
 // K3: one erasure pattern.  Indices fit a byte because classic codecs have at
