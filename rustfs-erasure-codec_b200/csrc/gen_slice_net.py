@@ -189,7 +189,7 @@ def main():
                 nets.append(net)
                 total += cost(*net)
             print(f"// GF(2^{bits}), nibble {q}: {total / 15:.1f} XOR instructions a network on average.")
-            for pairs in ((1, 2) if bits == 8 else (1,)):
+            for pairs in (1, 2):
                 emit_table(bits, q, pairs, nets)
 
 

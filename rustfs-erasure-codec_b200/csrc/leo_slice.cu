@@ -115,9 +115,9 @@ int slice_launch(int op, const SliceArgs &a, const SliceShape &sh, cudaStream_t 
   return cuda_status(cudaGetLastError());
 }
 
-// Tower coordinates of the element of each log value (exp: Cantor coordinates).
-void slice_elements(const uint16_t *exp, uint32_t order, uint16_t *out) {
-  for (uint32_t i = 0; i < order; ++i) out[i] = uint16_t(cantor_to_tower<8>(exp[i]));
+void slice_elements(int bits, const uint16_t *exp, uint32_t order, uint16_t *out) {
+  for (uint32_t i = 0; i < order; ++i)
+    out[i] = uint16_t(bits == 8 ? cantor_to_tower<8>(exp[i]) : cantor_to_tower<16>(exp[i]));
 }
 
 }  // namespace rsgpu

@@ -1,0 +1,351 @@
+// leo_slice16.cu -- launches of the bit-sliced Leopard GF(2^16) transforms
+// (slice16.cuh).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "codec.hpp"
+#include "launch_cfg.hpp"
+#include "leo_slice.hpp"
+#include "slice16.cuh"
+
+namespace rsgpu {
+
+#define RS_CUDA(expr)                              \
+  do {                                             \
+    cudaError_t e_ = (expr);                       \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
+  } while (0)
+
+namespace {
+
+
+// A work item of a launch: group `grp` of tile `x` of the chunk.
+struct Item16 {
+  uint32_t grp, x, job;
+  uint64_t col;
+};
+__device__ __forceinline__ Item16 item16(const Slice16Args &a, uint32_t it, uint32_t groups) {
+  Item16 w;
+  w.x = it / groups;
+  w.grp = it - w.x * groups;
+  const uint32_t tile = a.tile0 + w.x;
+  w.job = tile / a.tiles_per_job;
+  w.col = uint64_t(tile - w.job * a.tiles_per_job) * kRow16;
+  return w;
+}
+
+// What a warp needs of 32 consecutive lanes, lane l0 + t in thread t: all
+// looked up at once, then handed out by shuffles.
+struct Lanes16 {
+  uint64_t ptr;  // shard (0: nothing to do)
+  uint32_t c;    // tower constant of its scaling
+  // ROLE: 0 encode input, 1 decode input, 2 decode target, 3 parity output.
+  template <int ROLE>
+  __device__ __forceinline__ static Lanes16 get(const Slice16Args &a, const LeoJob &jd, uint32_t l) {
+    Lanes16 w{0, 0};
+    int sh = -1;
+    if (ROLE == 0) {
+      if (l < a.k) sh = int(l);
+    } else if (ROLE == 3) {
+      if (l < a.p) sh = int(a.k + l);
+    } else {
+      sh = l < a.p ? int(a.k + l) : l >= a.m && l < a.m + a.k ? int(l - a.m) : -1;
+      if (sh >= 0 && jd.role[sh] != ROLE) sh = -1;
+    }
+    if (sh >= 0) {
+      w.ptr = reinterpret_cast<uint64_t>(a.ptrs[jd.ptr_off + sh]);
+      if (ROLE == 1) w.c = a.elem[jd.err[l]];
+      if (ROLE == 2) w.c = a.elem[a.mod - jd.err[l]];
+    }
+    return w;
+  }
+  __device__ __forceinline__ Lanes16 at(uint32_t i) const {
+    return Lanes16{__shfl_sync(0xffffffffu, ptr, int(i)), __shfl_sync(0xffffffffu, c, int(i))};
+  }
+};
+
+// A: low IFFT of 2^bl consecutive lanes, shards -> V.  Decode: lane l is
+// parity l or data l - m, scaled by its locator.  Encode: lane l is data l,
+// at position m + l.
+template <bool DEC, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_slice16_a(Slice16Args a) {
+  extern __shared__ __align__(16) uint4 smem16[];
+  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
+  const uint32_t rows = 1u << a.bl;
+  const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem16)) + 16 * t;
+  const uint32_t groups = a.v_rows >> a.bl;
+#pragma unroll 1
+  for (uint32_t it = blockIdx.x; it < a.tiles * groups; it += gridDim.x) {
+    const Item16 w = item16(a, it, groups);
+    const LeoJob jd = a.jobs[w.job];
+    const uint32_t R = w.grp << a.bl, limit = DEC ? jd.input_count : a.k;
+    if (R >= limit) continue;  // CTA-uniform: zero lanes, never read
+    const Cols16 cols(w.col, t, a.len);
+#pragma unroll 1
+    for (uint32_t i0 = 0; i0 < rows; i0 += 32) {
+      const Lanes16 lanes = Lanes16::get<DEC ? 1 : 0>(a, jd, R + i0 + t);
+#pragma unroll 1
+      for (uint32_t i = warp; i < min(rows - i0, 32u); i += warps) {
+        const Lanes16 lane = lanes.at(i);
+        const uint32_t row = sbase + (i0 + i) * kRow16;
+        if (lane.ptr) {  // warp-uniform
+          uint32_t y[16];
+          cols.load(reinterpret_cast<const uint8_t *>(lane.ptr), y);
+          if (DEC) {
+            uint32_t x[16] = {};
+            mac16<4>(lane.c, x, y);
+            row16_store(row, x);
+          } else {
+            row16_store(row, y);
+          }
+        } else {
+          zero_row(row);
+        }
+      }
+    }
+    __syncthreads();
+    ifft16<3>(sbase, sbase, false, a.bl, DEC ? R : a.m + R, limit - R);
+    uint4 *out = a.v + (size_t(w.x) * a.v_rows + R) * 128 + t;
+#pragma unroll 1
+    for (uint32_t i = warp; i < rows; i += warps) copy_row_out(out + size_t(i) * 128, sbase + i * kRow16);
+    __syncthreads();
+  }
+}
+
+// B: the high layers of residue c (lanes c + 2^bl * j), V -> U.
+template <bool DEC, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_slice16_b(Slice16Args a) {
+  extern __shared__ __align__(16) uint4 smem16[];
+  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
+  const uint32_t rows = 1u << a.bh, residues = 1u << a.bl;
+  const uint32_t acc = uint32_t(__cvta_generic_to_shared(smem16)) + 16 * t, tmp = acc + rows * kRow16;
+#pragma unroll 1
+  for (uint32_t it = blockIdx.x; it < a.tiles * residues; it += gridDim.x) {
+    const Item16 w = item16(a, it, residues);
+    const uint4 *vin = a.v + (size_t(w.x) * a.v_rows + w.grp) * 128 + t;
+    uint4 *uout = a.u + (size_t(w.x) * a.u_rows + w.grp) * 128 + t;
+    const size_t step = size_t(residues) * 128;  // one j on
+    if (DEC) {
+      const uint32_t live = (a.jobs[w.job].input_count + residues - 1) >> a.bl;  // groups A wrote
+#pragma unroll 1
+      for (uint32_t j = warp; j < rows; j += warps) {
+        if (j < live)
+          copy_row_in(acc + j * kRow16, vin + j * step);
+        else
+          zero_row(acc + j * kRow16);
+      }
+      __syncthreads();
+      ifft16<2>(acc, acc, false, a.bh, 0, live);
+      derivative16<false>(acc, rows, nullptr);
+    } else {
+      const uint32_t groups = (a.k + a.m - 1) / a.m;
+#pragma unroll 1
+      for (uint32_t g = 0; g < groups; ++g) {
+        const uint32_t live = min(rows, ((a.k - g * a.m) + residues - 1) >> a.bl);
+        const uint32_t dst = g ? tmp : acc;
+#pragma unroll 1
+        for (uint32_t j = warp; j < rows; j += warps) {
+          if (j < live)
+            copy_row_in(dst + j * kRow16, vin + (g * rows + j) * step);
+          else
+            zero_row(dst + j * kRow16);
+        }
+        __syncthreads();
+        ifft16<2>(dst, acc, g != 0, a.bh, rows * (1 + g), live);
+      }
+    }
+    const uint32_t out = a.u_rows >> a.bl;
+    fft16<2>(acc, a.bh, 0, out, ~0u);
+#pragma unroll 1
+    for (uint32_t j = warp; j < out; j += warps) copy_row_out(uout + j * step, acc + j * kRow16);
+    __syncthreads();
+  }
+}
+
+// C: low FFT of 2^bl consecutive lanes, U (decode: plus N_low V) -> outputs.
+// MODE: 0 encode, 1 verify, 2 decode.
+template <int MODE, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_slice16_c(Slice16Args a) {
+  extern __shared__ __align__(16) uint4 smem16[];
+  __shared__ uint32_t s_need;
+  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
+  const uint32_t rows = 1u << a.bl;
+  const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem16)) + 16 * t;
+  const uint32_t groups = a.u_rows >> a.bl;
+#pragma unroll 1
+  for (uint32_t it = blockIdx.x; it < a.tiles * groups; it += gridDim.x) {
+    const Item16 w = item16(a, it, groups);
+    const LeoJob jd = a.jobs[w.job];
+    const uint32_t R = w.grp << a.bl;
+    uint32_t need = ~0u;
+    if (MODE == 2) {
+      // 4-lane blocks of the group that hold a target.
+      if (threadIdx.x < 32) {
+        uint32_t bits = 0;
+        for (uint32_t i = t; i < rows; i += 32) {
+          const uint32_t l = R + i;
+          const int sh = l < a.p ? int(a.k + l) : l >= a.m && l < a.m + a.k ? int(l - a.m) : -1;
+          if (sh >= 0 && jd.role[sh] == 2) bits |= 1u << (i >> 2);
+        }
+        bits = __reduce_or_sync(0xffffffffu, bits);
+        if (t == 0) s_need = bits;
+      }
+      __syncthreads();
+      need = s_need;
+      if (!need) {  // CTA-uniform
+        __syncthreads();  // s_need is read before the next item writes it
+        continue;
+      }
+    }
+    const uint4 *uin = a.u + (size_t(w.x) * a.u_rows + R) * 128 + t;
+    if (MODE == 2) {
+      const bool live = R < jd.input_count;
+      const uint4 *vin = a.v + (size_t(w.x) * a.v_rows + R) * 128 + t;
+      const uint4 *in = live ? vin : uin;
+#pragma unroll 2
+      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, in + size_t(i) * 128);
+      __syncthreads();
+      if (live) derivative16<true>(sbase, rows, uin);
+    } else {
+#pragma unroll 2
+      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, uin + size_t(i) * 128);
+      __syncthreads();
+    }
+    fft16<3>(sbase, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
+    const Cols16 cols(w.col, t, a.len);
+    uint32_t bad = 0;
+#pragma unroll 1
+    for (uint32_t i0 = 0; i0 < rows; i0 += 32) {
+      const Lanes16 lanes = Lanes16::get<MODE == 2 ? 2 : 3>(a, jd, R + i0 + t);
+#pragma unroll 1
+      for (uint32_t i = warp; i < min(rows - i0, 32u); i += warps) {
+        const Lanes16 lane = lanes.at(i);
+        if (!lane.ptr) continue;  // warp-uniform
+        uint8_t *out = reinterpret_cast<uint8_t *>(lane.ptr);
+        uint32_t v[16];
+        row16_load(sbase + (i0 + i) * kRow16, v);
+        if (MODE == 2) {
+          uint32_t x[16] = {};
+          mac16<4>(lane.c, x, v);
+          Cols16::bytes(x);
+          cols.store(out, x);
+        } else {
+          Cols16::bytes(v);
+          if (MODE == 1)
+            bad |= cols.compare(out, v);
+          else
+            cols.store(out, v);
+        }
+      }
+    }
+    if (MODE == 1 && __any_sync(0xffffffffu, bad) && t == 0) atomicOr(a.flags + jd.flag_idx, 1u);
+    __syncthreads();
+  }
+}
+
+using Kernel16 = void (*)(Slice16Args);
+struct Launch16 {
+  Kernel16 fn;
+  int threads;
+  size_t smem;
+  uint32_t groups;  // work items a tile
+};
+// Up to 32 rows (64 KiB): CTAs of 256 threads, one radix-4 group a warp, three
+// an SM at 80 registers.  64 rows: one CTA of 512.
+#define RS_PICK16(K, X) (smem <= 64 * 1024 ? K<X, 256, 2> : K<X, 512, 1>)
+void launches16(int op, const Slice16Args &a, Launch16 *out) {
+  const bool dec = op == RSGPU_OP_RECONSTRUCT;
+  auto fill = [&](int i, size_t smem, uint32_t groups, Kernel16 fn) {
+    out[i] = Launch16{fn, smem <= 64 * 1024 ? 256 : 512, smem, groups};
+  };
+  size_t smem = size_t(kRow16) << a.bl;
+  fill(0, smem, a.v_rows >> a.bl, dec ? RS_PICK16(k_slice16_a, true) : RS_PICK16(k_slice16_a, false));
+  fill(2, smem, a.u_rows >> a.bl, dec ? RS_PICK16(k_slice16_c, 2)
+                                  : op == RSGPU_OP_VERIFY ? RS_PICK16(k_slice16_c, 1) : RS_PICK16(k_slice16_c, 0));
+  smem = (size_t(kRow16) << a.bh) * (dec || a.k <= a.m ? 1 : 2);
+  fill(1, smem, 1u << a.bl, dec ? RS_PICK16(k_slice16_b, true) : RS_PICK16(k_slice16_b, false));
+}
+#undef RS_PICK16
+
+uint32_t log2u(uint32_t v) {
+  uint32_t b = 0;
+  while ((2u << b) <= v) ++b;
+  return b;
+}
+
+}  // namespace
+
+bool slice16_configure(int op, Slice16Args &a) {
+  const bool dec = op == RSGPU_OP_RECONSTRUCT;
+  const uint32_t b = log2u(dec ? a.n : a.m);
+  // Where this pays (one B200, register-stage / here, us):
+  //   rebuild 1024+512 16 KiB x 16 2424 / 1310, 300+100 671 / 370, 64+32 118 / 93,
+  //   48+16 (64 lanes) 65 / 65;  encode 2048+1024 1868 / 1134, 1024+512 732 / 550,
+  //   60+200 228 / 94, 512+128 231 / 252, 64+32 38 / 51
+  // One-level transforms in shared memory have no scratch traffic, and an
+  // encode of few lanes is little else.  Below 1 KiB a row is mostly empty.
+  if (b < (dec ? 7 : 8) || a.len < 1024) return false;
+  a.bl = dec ? b / 2 : std::max(b / 2, b > 5 ? b - 5 : 0u);
+  a.bh = b - a.bl;
+  if (a.bl > 6 || a.bh > 6) return false;
+  const uint32_t low = 1u << a.bl;
+  auto up = [&](uint32_t v) { return (v + low - 1) & ~(low - 1); };
+  a.v_rows = dec ? up(a.m + a.k) : up(a.k);
+  a.u_rows = dec ? up(a.m + a.k) : up(a.p);
+  // Positions of the constants (slice16.cuh).
+  const uint32_t top = dec ? a.n : a.m + (a.k + a.m - 1) / a.m * a.m;
+  if (top > 4096 || (top >> a.bl) > 256) return false;
+  a.tiles_per_job = uint32_t((a.len + kRow16 - 1) / kRow16);
+  return true;
+}
+
+static size_t tile_bytes16(const Slice16Args &a) { return (size_t(a.v_rows) + a.u_rows) * kRow16; }
+static uint64_t most_tiles16(const Slice16Args &a) { return std::max<uint64_t>(a.max_scratch / tile_bytes16(a), 1); }
+
+size_t slice16_scratch_limit(const Slice16Args &a) { return most_tiles16(a) * tile_bytes16(a); }
+
+size_t slice16_scratch_bytes(const Slice16Args &a, uint64_t tiles) {
+  const uint64_t chunks = (tiles + most_tiles16(a) - 1) / most_tiles16(a);
+  return size_t(chunks ? (tiles + chunks - 1) / chunks : 1) * tile_bytes16(a);
+}
+
+namespace {
+// Tiles of a chunk.
+uint32_t chunk16(const Slice16Args &a) {
+  return uint32_t(slice16_scratch_bytes(a, uint64_t(a.tiles_per_job) * a.n_jobs) / tile_bytes16(a));
+}
+}  // namespace
+
+uint64_t slice16_kernels(const Slice16Args &a) {
+  const uint32_t chunk = chunk16(a);
+  return 3 * ((uint64_t(a.tiles_per_job) * a.n_jobs + chunk - 1) / chunk);
+}
+
+int slice16_launch(int op, Slice16Args a, void *scratch, cudaStream_t s) {
+  Launch16 step[3];
+  launches16(op, a, step);
+  const uint64_t total = uint64_t(a.tiles_per_job) * a.n_jobs;
+  const uint32_t chunk = chunk16(a);
+  a.v = static_cast<uint4 *>(scratch);
+  a.u = a.v + size_t(chunk) * a.v_rows * (kRow16 / 16);
+  uint64_t launched = 0;
+  for (uint64_t t0 = 0; t0 < total; t0 += chunk) {
+    a.tile0 = uint32_t(t0);
+    a.tiles = uint32_t(std::min<uint64_t>(chunk, total - t0));
+    for (const Launch16 &l : step) {
+      const void *fn = reinterpret_cast<const void *>(l.fn);
+      RS_CUDA(ensure_smem_limit(fn, l.smem));
+      int per_sm = 0;
+      RS_CUDA(blocks_per_sm(fn, l.threads, l.smem, &per_sm));
+      const uint64_t items = uint64_t(a.tiles) * l.groups;
+      const int grid = int(std::min<uint64_t>(items, uint64_t(std::max(per_sm, 1)) * device_sm_count()));
+      l.fn<<<grid, l.threads, l.smem, s>>>(a);
+      ++launched;
+    }
+  }
+  launch_counter_add(launched);
+  return cuda_status(cudaGetLastError());
+}
+
+}  // namespace rsgpu

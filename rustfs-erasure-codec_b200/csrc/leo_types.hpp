@@ -2,6 +2,8 @@
 // the host runtime (leopard.cu, batch.cu) and the device code (leo_tile.cuh).
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace rsgpu {
@@ -55,6 +57,26 @@ struct SliceArgs {
   uint32_t k, p, m, n, mod;
   uint32_t wt;  // threads per row: a tile is 32 * wt bytes of every shard
   uint32_t rows;
+};
+
+// Launch of the bit-sliced GF(2^16) transforms (slice16.cuh): one chunk of
+// column tiles [tile0, tile0 + tiles) of all jobs' tiles.
+struct Slice16Args {
+  const LeoJob *jobs;
+  const uint8_t *const *ptrs;
+  uint32_t *flags;
+  const uint16_t *elem;  // per log value: the element's tower coordinates
+  uint64_t len;          // bytes per shard (multiple of 64)
+  uint32_t n_jobs;
+  uint32_t k, p, m, n, mod;
+  uint32_t bl, bh;       // low and high layers of the split
+  uint32_t tiles_per_job;
+  uint32_t tile0, tiles;
+  // Rows of a tile in each scratch buffer (multiples of 2^bl): V the low
+  // IFFT's lanes that can be non-zero, U the lanes an output needs.
+  uint32_t v_rows, u_rows;
+  uint64_t max_scratch;  // most bytes of both; more tiles go in equal chunks
+  uint4 *v, *u;
 };
 
 }  // namespace rsgpu

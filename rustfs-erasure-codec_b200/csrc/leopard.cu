@@ -150,7 +150,7 @@ struct LeoField {
   uint32_t *d_bank = nullptr;   // multiplier tables indexed by log value (half-warp layer kernels)
   uint32_t *d_kbank = nullptr;  // tables of the register-stage kernels (GF(2^8): 5+3 split; GF(2^16): 5+5+5+1)
   uint32_t *d_sktab = nullptr;  // d_kbank's entry of each skew entry: entry i holds the tables of log skew[i]
-  uint16_t *d_elem = nullptr;   // GF(2^8): tower coordinates of each log's element (slice_field.cuh)
+  uint16_t *d_elem = nullptr;   // tower coordinates of each log's element (slice_field.cuh)
   uint8_t *d_mul8 = nullptr;    // GF(2^8): products mul[a][b], 256 x 256 (device packing of dense maps)
   explicit LeoField(int b) : bits(b), host(b) {}
 };
@@ -213,10 +213,6 @@ static int leo_field(int bits, LeoField **out) {
         for (uint32_t b = 1; b < 256; ++b) mul[a * 256 + b] = uint8_t(t.exp[t.add_mod(t.log[a], t.log[b])]);
       RS_CUDA(cudaMalloc(&f->d_mul8, mul.size()));
       RS_CUDA(cudaMemcpy(f->d_mul8, mul.data(), mul.size(), cudaMemcpyHostToDevice));
-      std::vector<uint16_t> elem(t.order);
-      slice_elements(t.exp.data(), t.order, elem.data());
-      RS_CUDA(cudaMalloc(&f->d_elem, elem.size() * 2));
-      RS_CUDA(cudaMemcpy(f->d_elem, elem.data(), elem.size() * 2, cudaMemcpyHostToDevice));
     } else {
       // Per log value, 32 lanes x 4 words (layout of leo_fft.cuh): c * i,
       // c * (i << 5), c * (i << 10) for i = lane, and c * 2^15, each
@@ -236,6 +232,10 @@ static int leo_field(int bits, LeoField **out) {
       RS_CUDA(cudaMalloc(&f->d_sktab, sk.size() * 4));
       RS_CUDA(cudaMemcpy(f->d_sktab, sk.data(), sk.size() * 4, cudaMemcpyHostToDevice));
     }
+    std::vector<uint16_t> elem(t.order);
+    slice_elements(bits, t.exp.data(), t.order, elem.data());
+    RS_CUDA(cudaMalloc(&f->d_elem, elem.size() * 2));
+    RS_CUDA(cudaMemcpy(f->d_elem, elem.data(), elem.size() * 2, cudaMemcpyHostToDevice));
     fields[slot] = f;
   }
   *out = fields[slot];
@@ -488,6 +488,13 @@ struct LeoLaunch {
   LeoArgs args{};
   SliceArgs slice{};
   SliceShape slice_shape;
+  // Bit-sliced GF(2^16) kernels (leo_slice16.cu), with the rows that pass
+  // between them in own_scratch or scratch16 (the codec's slab when the launch
+  // was built).  A launch under stream capture runs the engine's kernels
+  // instead: replays could overlap on the slab, and theirs need none (encode).
+  bool sliced16 = false;
+  Slice16Args slice16{};
+  void *scratch16 = nullptr;
   void *d_blob = nullptr;  // jobs | pointers | roles
   // One-shot launches allocate the blob on their stream and free it there
   // after the kernel; prepared launches own it until destroyed.
@@ -1018,11 +1025,35 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
   a.sktab = st.field->d_sktab;
   fill_stages(a);
   L.engine = leo_engine();
+  // The bit-sliced kernels read shards 16 bytes at a time; other pointers
+  // stay on the register-stage kernels' 4-byte accesses.
+  uintptr_t low = 0;
+  for (size_t i = 0; i < n_stripes * total; ++i) low |= reinterpret_cast<uintptr_t>(shards[i]);
+  if (L.engine == 1 && st.field->bits == 16 && (low & 15) == 0) {
+    Slice16Args &sa = L.slice16;
+    sa.jobs = a.jobs;
+    sa.ptrs = a.ptrs;
+    sa.flags = flags;
+    sa.elem = st.field->d_elem;
+    sa.len = len;
+    sa.n_jobs = a.n_jobs;
+    sa.k = a.k;
+    sa.p = a.p;
+    sa.m = a.m;
+    sa.n = a.n;
+    sa.mod = a.mod;
+    sa.max_scratch = L.own_scratch ? kStreamScratch16 : kSlabScratch16;
+    if (slice16_configure(op, sa)) {
+      L.sliced16 = true;
+      if (!L.own_scratch) {
+        int rc = grow_scratch(st, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs));
+        if (rc) return rc;
+        std::lock_guard<std::mutex> g(st.scratch_mu);
+        L.scratch16 = st.scratch;
+      }
+    }
+  }
   if (L.engine == 1 && st.field->bits == 8) {
-    // The bit-sliced kernels read shards 16 bytes at a time; other pointers
-    // stay on the register-stage kernels' 4-byte accesses.
-    uintptr_t low = 0;
-    for (size_t i = 0; i < n_stripes * total; ++i) low |= reinterpret_cast<uintptr_t>(shards[i]);
     if ((low & 15) == 0 && slice_pays(op, a.k, a.m, a.n, uint64_t(len) * a.n_jobs)) {
       L.engine = 2;
       SliceArgs &sa = L.slice;
@@ -1086,7 +1117,9 @@ int leo_launch_kernel(const LeoLaunch &L, cudaStream_t s);
 // capture cannot be waited on inside it).
 int leo_launch(const LeoLaunch &L, cudaStream_t s) {
   if (L.args.n_jobs == 0) return RSGPU_OK;
-  if (!L.global_work || L.own_scratch) return leo_launch_kernel(L, s);
+  const int op = L.decode ? RSGPU_OP_RECONSTRUCT : L.verify ? RSGPU_OP_VERIFY : RSGPU_OP_ENCODE;
+  if (L.sliced16 && L.own_scratch) return slice16_launch(op, L.slice16, L.own_scratch, s);
+  if (!L.sliced16 && (!L.global_work || L.own_scratch)) return leo_launch_kernel(L, s);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   RS_CUDA(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) return leo_launch_kernel(L, s);
@@ -1094,7 +1127,7 @@ int leo_launch(const LeoLaunch &L, cudaStream_t s) {
   std::lock_guard<std::mutex> g(st.scratch_mu);
   if (!st.scratch_done) RS_CUDA(cudaEventCreateWithFlags(&st.scratch_done, cudaEventDisableTiming));
   RS_CUDA(cudaStreamWaitEvent(s, st.scratch_done, 0));
-  int rc = leo_launch_kernel(L, s);
+  int rc = L.sliced16 ? slice16_launch(op, L.slice16, L.scratch16, s) : leo_launch_kernel(L, s);
   if (rc) return rc;
   return cuda_status(cudaEventRecord(st.scratch_done, s));
 }
@@ -1166,7 +1199,10 @@ int leo_launch_kernel(const LeoLaunch &L, cudaStream_t s) {
 }
 }  // namespace
 
-uint32_t leo_kernel_count(const LeoLaunch &L) { return L.args.n_jobs ? 1 : 0; }
+uint32_t leo_kernel_count(const LeoLaunch &L) {
+  if (!L.args.n_jobs) return 0;
+  return L.sliced16 ? uint32_t(slice16_kernels(L.slice16)) : 1;
+}
 
 int prepare_other(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const uint8_t *present, size_t len,
                   int goal, uint32_t *flags, std::shared_ptr<LeoLaunch> &out) {
@@ -1178,12 +1214,25 @@ int prepare_other(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, co
   return RSGPU_OK;
 }
 
-// Work rows of a full grid of the decode kernel when they live in global
-// memory (configure_fft: n rows of two 64-byte blocks per CTA, beyond
-// 200 KiB of shared memory); 0 when they fit shared memory.
+// Scratch of any reconstruction launch of the codec: the register-stage
+// kernel's work rows when they live in global memory (configure_fft: n rows of
+// two 64-byte blocks per CTA, beyond 200 KiB of shared memory), or the
+// bit-sliced GF(2^16) kernels' rows; 0 when neither needs any.
 size_t leo_reconstruct_scratch_bytes(Codec &c) {
   const size_t rows = c.leo->n, per_cta = rows * 2 * 64;
-  return per_cta > 200 * 1024 ? size_t(kGlobalBlocks) * sm_count() * per_cta : 0;
+  size_t need = per_cta > 200 * 1024 ? size_t(kGlobalBlocks) * sm_count() * per_cta : 0;
+  if (c.leo->field->bits == 16) {
+    Slice16Args a{};
+    a.k = uint32_t(c.k);
+    a.p = uint32_t(c.m);
+    a.m = c.leo->m;
+    a.n = c.leo->n;
+    a.len = size_t(1) << 20;
+    a.n_jobs = 1;
+    a.max_scratch = kStreamScratch16;
+    if (slice16_configure(RSGPU_OP_RECONSTRUCT, a)) need = std::max(need, slice16_scratch_limit(a));
+  }
+  return need;
 }
 
 void leo_set_scratch(LeoLaunch &L, void *scratch) {
