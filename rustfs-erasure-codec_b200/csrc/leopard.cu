@@ -472,8 +472,8 @@ struct LeopardState {
   ~LeopardState() {
     cudaDeviceSynchronize();
     for (void *p : plan_slabs) cudaFree(p);
-    if (scratch) cudaFree(scratch);
-    for (void *p : owned) cudaFree(p);
+    if (scratch) cudaFreeAsync(scratch, cudaStreamPerThread);  // back to the library's pool
+    for (void *p : owned) cudaFreeAsync(p, cudaStreamPerThread);
     if (d_dense_enc) cudaFree(d_dense_enc);
     if (scratch_done) cudaEventDestroy(scratch_done);
   }
@@ -519,14 +519,22 @@ struct LeoLaunch {
 
 // Grow the codec's scratch slab to `need` bytes.  A slab another thread may
 // still have in a built launch is retired (kept until the codec is
-// destroyed), never freed under it.
+// destroyed), never freed under it.  Slabs come from the library's pool, which
+// keeps what a destroyed codec gave back: mapping 256 MiB afresh took 2 ms of a
+// codec's first launch.
 int grow_scratch(LeopardState &st, size_t need) {
   std::lock_guard<std::mutex> g(st.scratch_mu);
   if (st.scratch_bytes >= need) return RSGPU_OK;
   if (st.scratch) st.owned.push_back(st.scratch);
   st.scratch = nullptr;
   st.scratch_bytes = 0;
-  RS_CUDA(cudaMalloc(&st.scratch, need));
+  RS_CUDA(cudaError_t(lib_malloc_async(&st.scratch, need, cudaStreamPerThread)));
+  const cudaError_t e = cudaStreamSynchronize(cudaStreamPerThread);  // usable on any stream from here
+  if (e != cudaSuccess) {
+    cudaFreeAsync(st.scratch, cudaStreamPerThread);
+    st.scratch = nullptr;
+    return cuda_status(e);
+  }
   st.scratch_bytes = need;
   return RSGPU_OK;
 }
