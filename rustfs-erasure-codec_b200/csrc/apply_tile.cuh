@@ -293,7 +293,7 @@ __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t 
             if (VERIFY) {
               uint4 e = ld_stream(dst);
               bad |= (e.x != o[r][0]) | (e.y != o[r][1]) | (e.z != o[r][2]) | (e.w != o[r][3]);
-              if (d.verify_store)
+              if (d.mode & kJobStore)
                 st_stream(const_cast<uint8_t *>(ptr[n_in + d.n_out + out]) + col[v],
                           make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]));
             } else if (ACC) {
@@ -332,7 +332,7 @@ __device__ __forceinline__ bool apply_column(const uint8_t *const *ptrs, const J
       const uint8_t b = uint8_t(acc >> (8 * r));
       if (VERIFY) {
         bad |= (*dst != b);
-        if (d.verify_store) const_cast<uint8_t *>(ptr[d.n_in + d.n_out + g * 4 + r])[col] = b;
+        if (d.mode & kJobStore) const_cast<uint8_t *>(ptr[d.n_in + d.n_out + g * 4 + r])[col] = b;
       } else if (ACC)
         *dst ^= b;
       else

@@ -447,17 +447,25 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   verify = vfy;
   max_tail = 0;
   uint32_t max_out = 0, uni_in = jobs.empty() ? 0 : jobs[0].n_in;
-  int any_vec = 0;
+  int any_vec = 0, any_unaligned = 0;
+  // Misaligned jobs: by words from about here, one thread a byte column below
+  // (10+4 at 5001 bytes, one stripe: 8 against 13 us; 1029 bytes x 1000: 21
+  // both; 12+4 at 100003 x 128: 351 against 103).
+  const bool words = uint64_t(len) * jobs.size() >= (256u << 10);
   int tbl_stage = 0;
   for (auto &j : jobs) {
     tbl_stage |= j.tbl != jobs[0].tbl;
     if (j.n_in != uni_in) uni_in = 0;
     bool aligned = true;
-    const uint32_t n_ptr = uint32_t(j.n_in) + j.n_out * (j.verify_store ? 2u : 1u);
+    const uint32_t n_ptr = uint32_t(j.n_in) + j.n_out * (j.mode & kJobStore ? 2u : 1u);
     for (uint32_t i = 0; i < n_ptr; ++i)
       aligned &= (reinterpret_cast<uintptr_t>(ptrs[j.ptr_off + i]) & 15) == 0;
     j.vec_len = aligned ? (len & ~uint64_t(15)) : 0;
-    max_tail = std::max<uint64_t>(max_tail, len - j.vec_len);
+    if (aligned || !words)
+      max_tail = std::max<uint64_t>(max_tail, len - j.vec_len);
+    else
+      j.mode |= kJobUnaligned;
+    any_unaligned |= !aligned && words;
     max_out = std::max<uint32_t>(max_out, j.n_out);
     any_vec |= j.vec_len > 0;
   }
@@ -481,6 +489,7 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   args.max_out = max_out;
   args.uni_in = uni_in;
   args.any_vec = any_vec;
+  args.any_unaligned = any_unaligned;
   args.tbl_stage = tbl_stage;
   args.accumulate = accumulate ? 1 : 0;
   return RSGPU_OK;
@@ -604,7 +613,7 @@ int Codec::verify_with_buffer_dev(uint8_t *const *ptrs3, size_t len, uint8_t *ok
   jobs[0].ptr_off = 0;
   jobs[0].n_in = uint16_t(k);
   jobs[0].n_out = uint16_t(m);
-  jobs[0].verify_store = 1;
+  jobs[0].mode = kJobStore;
   jobs[0].tbl = d_enc_tbl;
   std::vector<const uint8_t *> ptrs(ptrs3, ptrs3 + k + 2 * m);
   uint32_t *flags = nullptr;

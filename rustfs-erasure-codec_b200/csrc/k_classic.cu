@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a
               if (VERIFY) {
                 const uint4 e = lds128(slot0 + r * kSlot + v * kApplyThreads * kApplyVec);
                 bad |= (e.x != o[r][0]) | (e.y != o[r][1]) | (e.z != o[r][2]) | (e.w != o[r][3]);
-                if (d.verify_store)
+                if (d.mode & kJobStore)
                   st_stream(const_cast<uint8_t *>(a.ptrs[d.ptr_off + n_in + d.n_out + r]) + col[v],
                             make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]));
               } else {
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBloc
       const uint8_t *const *out = a.ptrs + d.ptr_off + K + (VERIFY ? d.n_out : 0);
 #pragma unroll
       for (int r = 0; r < 4; ++r)
-        dst[r] = uint32_t(r) < d.n_out && (!VERIFY || d.verify_store) ? const_cast<uint8_t *>(out[r]) : nullptr;
+        dst[r] = uint32_t(r) < d.n_out && (!VERIFY || (d.mode & kJobStore)) ? const_cast<uint8_t *>(out[r]) : nullptr;
       if (d.tbl != cur) {
         lut.load(d.tbl, lane);
         cur = d.tbl;
@@ -437,8 +437,180 @@ __global__ void k_apply_tail(ApplyArgs a, uint64_t max_tail) {
     const uint32_t job = uint32_t(i / max_tail);
     const JobDesc d = a.jobs[job];
     const uint64_t col = d.vec_len + (i - uint64_t(job) * max_tail);
-    if (col >= a.len) continue;
+    if (col >= a.len || (d.mode & kJobUnaligned)) continue;
     if (apply_column<VERIFY, ACC>(a.ptrs, d, col) && VERIFY) atomicOr(a.flags + d.flag_idx, 1u);
+  }
+}
+
+// ------------------------------------------------------------------ K1, any alignment
+// Jobs whose pointers are not all 16-byte aligned (shards of odd length packed
+// back to back, for one), any number of inputs and outputs.  A thread takes
+// kWordsU words of four columns, 128 bytes of consecutive words a warp; an
+// input word at an odd address is put together from the two aligned words
+// around it, an output word is written as the aligned word that overlaps it
+// most (its neighbour's bytes come by a shuffle) with single bytes at the ends
+// of a warp's run.  The columns covered this way, 4 to 4 + 4 * n, keep every
+// aligned word inside the shard; the few before and after are the work of an
+// extra warp.  The alternative for such jobs was one thread a byte
+// column: verify of 128 12+4 stripes of 100003 bytes
+// 351 -> 103 us, encode 264 -> 115, 24+4 at 50001 bytes x 100 encode 174 -> 77.
+constexpr int kWordsU = 4;
+constexpr uint32_t kTileU = kApplyThreads * 4 * kWordsU;
+
+// Words of a thread's columns from p on (word v at p + v * kApplyThreads * 4),
+// zero where !on.  Both aligned words are read even when one would do: without
+// the branch all loads are in flight together, and columns 4 .. 4 + 4 * n keep
+// both inside the shard.
+__device__ __forceinline__ void ldg_words(const uint8_t *p, const bool *on, uint32_t *x) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3));
+  const uint32_t sh = 8 * uint32_t(at & 3);
+  uint32_t lo[kWordsU], hi[kWordsU];
+#pragma unroll
+  for (int v = 0; v < kWordsU; ++v) {
+    lo[v] = on[v] ? __ldg(w + v * kApplyThreads) : 0;
+    hi[v] = on[v] ? __ldg(w + v * kApplyThreads + 1) : 0;
+  }
+#pragma unroll
+  for (int v = 0; v < kWordsU; ++v) x[v] = __funnelshift_r(lo[v], hi[v], sh);
+}
+
+// Writes (ACC: XORs) the warp's words v at p (this lane's address); `on` lanes
+// are a prefix of the warp.
+template <bool ACC>
+__device__ __forceinline__ void stg_words(uint8_t *p, uint32_t v, bool on, uint32_t lane) {
+  const uint32_t sh = uint32_t(reinterpret_cast<uintptr_t>(p) & 3);  // uniform
+  const uint32_t prev = __shfl_up_sync(0xffffffffu, v, 1);
+  const uint32_t active = __ballot_sync(0xffffffffu, on);
+  if (!on) return;
+  uint8_t *w = p - sh;
+  if (sh == 0 || lane) {
+    const uint32_t out = sh ? __funnelshift_l(prev, v, 8 * sh) : v;
+    uint32_t *dst = reinterpret_cast<uint32_t *>(w);
+    *dst = ACC ? (*dst ^ out) : out;
+  } else {
+    for (uint32_t b = 0; b < 4 - sh; ++b) p[b] = uint8_t(v >> (8 * b)) ^ (ACC ? p[b] : uint8_t(0));
+  }
+  if (sh && lane == 31u - __clz(active))
+    for (uint32_t b = 4 - sh; b < 4; ++b) p[b] = uint8_t(v >> (8 * b)) ^ (ACC ? p[b] : uint8_t(0));
+}
+
+template <int C>
+__device__ __forceinline__ void unaligned_mac(uint32_t (*acc)[4], const uint8_t *const *ptr, const uint32_t *tbl,
+                                              uint64_t col, const bool *on, uint32_t live, uint32_t lane) {
+  Lut<C> lut;
+  lut_load<C>(lut, lane, [&](int i, uint32_t w) { return __ldg(tbl + i * kTableWords + w); });
+  uint32_t x[C][kWordsU];
+#pragma unroll
+  for (int i = 0; i < C; ++i) ldg_words(ptr[i] + col, on, x[i]);
+#pragma unroll
+  for (int v = 0; v < kWordsU; ++v) {
+    if (uint32_t(v) >= live) break;  // CTA-uniform
+    uint32_t y[C], m[Lut<C>::kMixed];
+#pragma unroll
+    for (int i = 0; i < C; ++i) y[i] = x[i][v];
+    lut_index<C>(y, m);
+    lut_mac<C>(lut, y, m, acc[v]);
+  }
+}
+
+template <bool VERIFY, bool ACC>
+__global__ void __launch_bounds__(kApplyThreads + 32, 3) k_apply_unaligned(ApplyArgs a) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint64_t words = a.len >= 12 ? (a.len - 8) / 4 : 0;
+  const uint32_t tiles_per_job = uint32_t((words * 4 + kTileU - 1) / kTileU) + (words ? 0 : 1);
+  const uint32_t total = tiles_per_job * a.n_jobs;
+  for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const uint32_t job = t / tiles_per_job, tile = t - job * tiles_per_job;
+    const JobDesc d = a.jobs[job];
+    if (!(d.mode & kJobUnaligned)) continue;  // CTA-uniform
+    const uint8_t *const *ptr = a.ptrs + d.ptr_off;
+    if (tid >= kApplyThreads) {
+      // The last warp, beside the others' words: the at most 11 columns before
+      // and after them, two threads each, with the job's first tile.
+      if (tile) continue;
+      const uint64_t head = a.len < 4 ? a.len : 4, rest = a.len - head - 4 * words;
+      const uint32_t e = lane >> 1;
+      const bool mine = e < head + rest;
+      const uint64_t c = e < head ? e : 4 * words + e;
+      bool bad = false;
+      for (uint32_t g = 0; g * 4 < d.n_out; ++g) {
+        uint32_t acc = 0;
+        if (mine) {
+          const uint32_t *tbl = d.tbl + size_t(g) * d.n_in * kTableWords;
+#pragma unroll 4
+          for (uint32_t j = lane & 1; j < d.n_in; j += 2) {
+            const uint32_t x = ptr[j][c];
+            acc ^= __ldg(tbl + j * kTableWords + (x & 15)) ^ __ldg(tbl + j * kTableWords + 16 + (x >> 4));
+          }
+        }
+        acc ^= __shfl_xor_sync(0xffffffffu, acc, 1);
+#pragma unroll
+        for (uint32_t q = 0; q < 2; ++q) {
+          const uint32_t r = 2 * (lane & 1) + q, out = 4 * g + r;
+          if (mine && out < d.n_out) {
+            const uint8_t b = uint8_t(acc >> (8 * r));
+            uint8_t *dst = const_cast<uint8_t *>(ptr[d.n_in + out]) + c;
+            if (VERIFY) {
+              bad |= *dst != b;
+              if (d.mode & kJobStore) const_cast<uint8_t *>(ptr[d.n_in + d.n_out + out])[c] = b;
+            } else {
+              *dst = ACC ? uint8_t(*dst ^ b) : b;
+            }
+          }
+        }
+      }
+      if (VERIFY && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags + d.flag_idx, 1u);
+      continue;
+    }
+    if (!words) continue;
+    const uint64_t word = uint64_t(tile) * (kTileU / 4) + tid, col = 4 + 4 * word;
+    const uint64_t left = words - uint64_t(tile) * (kTileU / 4);
+    const uint32_t live = uint32_t(left >= kTileU / 4 ? kWordsU : (left + kApplyThreads - 1) / kApplyThreads);
+    bool on[kWordsU], bad = false;
+#pragma unroll
+    for (int v = 0; v < kWordsU; ++v) on[v] = word + v * kApplyThreads < words;
+    for (uint32_t g = 0; g * 4 < d.n_out; ++g) {
+      uint32_t acc[kWordsU][4];
+#pragma unroll
+      for (int v = 0; v < kWordsU; ++v)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[v][i] = 0;
+      const uint32_t *tbl = d.tbl + size_t(g) * d.n_in * kTableWords;
+      uint32_t j = 0;
+#pragma unroll 1
+      for (; j + 5 <= d.n_in; j += 5) unaligned_mac<5>(acc, ptr + j, tbl + j * kTableWords, col, on, live, lane);
+      if (j + 3 <= d.n_in) {
+        unaligned_mac<3>(acc, ptr + j, tbl + j * kTableWords, col, on, live, lane);
+        j += 3;
+      }
+#pragma unroll 1
+      for (; j < d.n_in; ++j) unaligned_mac<1>(acc, ptr + j, tbl + j * kTableWords, col, on, live, lane);
+#pragma unroll
+      for (int v = 0; v < kWordsU; ++v) {
+        uint32_t o[4];
+        transpose4(acc[v], o);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[v][r] = o[r];
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t out = 4 * g + r;
+        if (out >= d.n_out) break;  // CTA-uniform
+        uint8_t *dst = const_cast<uint8_t *>(ptr[d.n_in + out]) + col;
+        if (VERIFY) {
+          uint32_t have[kWordsU];
+          ldg_words(dst, on, have);
+#pragma unroll
+          for (int v = 0; v < kWordsU; ++v) bad |= on[v] && have[v] != acc[v][r];
+          if (!(d.mode & kJobStore)) continue;
+          dst = const_cast<uint8_t *>(ptr[d.n_in + d.n_out + out]) + col;
+        }
+#pragma unroll
+        for (int v = 0; v < kWordsU; ++v) stg_words<ACC>(dst + v * kApplyThreads * 4, acc[v][r], on[v], lane);
+      }
+    }
+    if (VERIFY && __any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags + d.flag_idx, 1u);
   }
 }
 
@@ -655,6 +827,15 @@ void launch_reg_k(const ApplyArgs &a, cudaStream_t s) {
   }
 }
 
+template <bool VERIFY, bool ACC>
+void launch_unaligned(const ApplyArgs &a, cudaStream_t s) {
+  static int grid_max = 0;
+  if (!grid_max) grid_max = grid_for((const void *)k_apply_unaligned<VERIFY, ACC>, kApplyThreads + 32, 0);
+  const uint64_t tiles = (a.len + kTileU - 1) / kTileU * a.n_jobs;
+  const int grid = int(tiles < uint64_t(grid_max) ? tiles : grid_max);
+  k_apply_unaligned<VERIFY, ACC><<<grid, kApplyThreads + 32, 0, s>>>(a);
+}
+
 // More than 4 outputs: the register-path tile, 8 outputs a pass.  At most 4:
 // tables in registers up to kRegInputs inputs a job (beyond, they no longer
 // fit), the staged tile with tables read per step for wider jobs and for
@@ -697,6 +878,15 @@ cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cud
       launch_write_or_verify<true>(a, apply_variant(), s);
     else
       launch_write_or_verify<false>(a, apply_variant(), s);
+    ++launches;
+  }
+  if (a.any_unaligned) {
+    if (a.accumulate)
+      launch_unaligned<false, true>(a, s);
+    else if (verify)
+      launch_unaligned<true, false>(a, s);
+    else
+      launch_unaligned<false, false>(a, s);
     ++launches;
   }
   if (max_tail) {

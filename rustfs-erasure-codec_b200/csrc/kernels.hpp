@@ -17,6 +17,7 @@ struct ApplyArgs {
   uint32_t max_out;             // largest n_out over the jobs
   uint32_t uni_in;              // n_in of every job, 0 when they differ
   int any_vec;                  // some job has vec_len > 0
+  int any_unaligned;            // some job is kJobUnaligned
   int accumulate;               // outputs ^= products (incremental parity update)
   uint32_t *stall;              // device status word: a bounded wait of the TMA-staged tile ran out (may be null)
   int tbl_stage;                // jobs carry different tables: the TMA-staged tile copies them with the data
