@@ -306,8 +306,9 @@ struct MixBatch {
   cudaGraphExec_t exec = nullptr;
   rsgpu_mix_info info{};
   std::vector<uint32_t *> owned_tables;  // private copies of classic decode tables
-  // One-shot batches: wide Leopard reconstructions run by their codec's own
-  // decode kernel, launched on the batch's stream after k_mix.
+  // Launches after k_mix on the batch's stream: bit-sliced Leopard GF(2^8)
+  // operations, and in one-shot batches wide Leopard reconstructions run by
+  // their codec's own decode kernel.
   std::vector<std::shared_ptr<LeoLaunch>> side;
   uint32_t mix_kernels = 0;  // k_mix launches per launch (0 or 1)
   std::vector<void *> ordered_bufs;  // one-shot batches: dense maps derived on the stream
@@ -525,6 +526,48 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
       if (rc) return rc;
       routed[i] = size_t(fft_rows(g, ops[i].op)) * 2 * 64 > kMixSmem;
     }
+  // Leopard GF(2^8) operations that the bit-sliced kernels run faster go in
+  // one launch per (codec, operation, goal) beside k_mix (planners TABLE and
+  // MODEL; the fixed rule and forced plans stay in k_mix).  Encodes and
+  // verifies always; rebuilds unless the dense map in k_mix takes less: its
+  // time goes with present * ceil(targets / 4), theirs with lanes * layers.
+  // One B200, 8 stripes of 512 KiB shards, dense map / bit-sliced, us:
+  //   rebuild 128+64, 4 lost 314 / 1013, 16 lost 867 / 1082, 24 lost 1232 / 1098, 64 lost 2486 / 1142
+  //   rebuild 32+16, 4 lost 83 / 202, 16 lost 169 / 216;  60+20, 16 lost 322 / 521
+  //   encode 128+64 2419 (FFT in k_mix 984) / 487, 32+16 182 / 91, 20+8 61 / 55
+  std::vector<char> sliced(n_ops, 0);
+  if (!forced && opt.planner != RSGPU_PLANNER_FIXED) {
+    constexpr uint64_t kSlicedMinColumns = 256 << 10;  // below, a launch of its own does not pay
+    std::map<std::tuple<const Codec *, int>, uint64_t> columns;
+    for (int pass = 0; pass < 2; ++pass)
+      for (size_t i = 0; i < n_ops; ++i) {
+        Codec &c = const_cast<rsgpu_codec *>(ops[i].codec)->c;
+        if (c.family != RSGPU_FAMILY_LEOPARD_GF8 || routed[i]) continue;
+        LeoGeometry g{};
+        int rc = leopard_geometry(c, &g);
+        if (rc) return rc;
+        uintptr_t low = 0;
+        uint64_t present = 0, targets = 0, layers = 0;
+        for (size_t x = 0; x < c.k + c.m; ++x) {
+          low |= reinterpret_cast<uintptr_t>(ops[i].shards[x]);
+          if (ops[i].op != RSGPU_OP_RECONSTRUCT) continue;
+          present += ops[i].present[x] ? 1 : 0;
+          targets += !ops[i].present[x] && (ops[i].goal == RSGPU_GOAL_ALL || x < c.k);
+        }
+        if (low & 15) continue;
+        if (ops[i].op == RSGPU_OP_RECONSTRUCT) {
+          while ((1u << layers) < g.n) ++layers;
+          if (!targets || present * ((targets + 3) / 4) * 22 <= g.n * layers * 10) continue;
+        }
+        uint64_t &sum = columns[std::make_tuple(&ops[i].codec->c, int(ops[i].op))];
+        if (pass == 0)
+          sum += ops[i].shard_len;
+        else if (sum >= kSlicedMinColumns && leo_slice_takes(c, ops[i].op, sum)) {
+          sliced[i] = 1;
+          b.plans[i] = mix_default_plan(c, ops[i].op, ops[i].shard_len);
+        }
+      }
+  }
   // One-shot batches run large Leopard GF(2^8) rebuilds whose dense map is
   // not cached through a map derived on the batch's stream (the FFT decode
   // of unit vectors, then a packing kernel; no host wait) instead of the FFT
@@ -538,7 +581,7 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
     for (size_t i = 0; i < n_ops; ++i) {
       Codec &c = const_cast<rsgpu_codec *>(ops[i].codec)->c;
       if (c.family != RSGPU_FAMILY_LEOPARD_GF8 || ops[i].op != RSGPU_OP_RECONSTRUCT ||
-          b.plans[i].algo != RSGPU_ALGO_FFT || routed[i])
+          b.plans[i].algo != RSGPU_ALGO_FFT || routed[i] || sliced[i])
         continue;
       inline_dense[i] = uint64_t(c.k + c.m) * ops[i].shard_len >= kInlineDenseBytes;
     }
@@ -554,7 +597,7 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
   std::map<const Codec *, std::vector<size_t>> leo_fft_rec;
   for (size_t i = 0; i < n_ops; ++i) {
     const Codec &c = ops[i].codec->c;
-    if (ops[i].op != RSGPU_OP_RECONSTRUCT || routed[i] || inline_dense[i]) continue;
+    if (ops[i].op != RSGPU_OP_RECONSTRUCT || routed[i] || inline_dense[i] || sliced[i]) continue;
     if (!is_leopard(c))
       classic_rec[&c].push_back(i);
     else if (b.plans[i].algo == RSGPU_ALGO_APPLY)
@@ -653,7 +696,7 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
   std::map<const Codec *, size_t> dense_enc_tbl;  // word offset into B.tables
   for (size_t i = 0; i < n_ops; ++i) {
     const Codec &c = ops[i].codec->c;
-    if (!is_leopard(c) || b.plans[i].algo != RSGPU_ALGO_APPLY || ops[i].op == RSGPU_OP_RECONSTRUCT) continue;
+    if (!is_leopard(c) || b.plans[i].algo != RSGPU_ALGO_APPLY || ops[i].op == RSGPU_OP_RECONSTRUCT || sliced[i]) continue;
     if (dense_enc_tbl.count(&c)) continue;
     std::vector<uint8_t> rows;
     int rc = leopard_dense_encode(const_cast<Codec &>(c), rows);
@@ -730,7 +773,7 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
 
   // ---- jobs
   for (size_t i = 0; i < n_ops; ++i) {
-    if (routed[i]) continue;
+    if (routed[i] || sliced[i]) continue;
     const rsgpu_mix_op &o = ops[i];
     if (inline_dense[i]) {
       const InlineMap &mp = imaps[i];
@@ -925,6 +968,46 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
     RS_CUDA(cudaMemsetAsync(b.d_flags, 0, std::max<size_t>(n_ops, 1) * 4, b.stream));
   else
     RS_CUDA(cudaMemset(b.d_flags, 0, std::max<size_t>(n_ops, 1) * 4));
+  // ---- bit-sliced launches, one per (codec, operation, goal)
+  size_t sliced_jobs = 0;
+  {
+    std::map<std::tuple<const Codec *, int, int>, std::vector<size_t>> groups;
+    for (size_t i = 0; i < n_ops; ++i)
+      if (sliced[i])
+        groups[std::make_tuple(&ops[i].codec->c, int(ops[i].op),
+                               ops[i].op == RSGPU_OP_RECONSTRUCT ? int(ops[i].goal) : 0)].push_back(i);
+    for (auto &kv : groups) {
+      Codec &c = const_cast<Codec &>(*std::get<0>(kv.first));
+      const int op = std::get<1>(kv.first);
+      const size_t total = c.k + c.m;
+      std::vector<uint8_t *> sh;
+      std::vector<uint8_t> pres;
+      std::vector<size_t> lens;
+      std::vector<uint32_t> flag_of;
+      // Longest stripes first: the last work items are then the short ones.
+      std::stable_sort(kv.second.begin(), kv.second.end(),
+                       [&](size_t x, size_t y) { return ops[x].shard_len > ops[y].shard_len; });
+      for (size_t i : kv.second) {
+        sh.insert(sh.end(), ops[i].shards, ops[i].shards + total);
+        lens.push_back(ops[i].shard_len);
+        flag_of.push_back(uint32_t(i));
+        size_t moved = total;
+        if (op == RSGPU_OP_RECONSTRUCT) {
+          pres.insert(pres.end(), ops[i].present, ops[i].present + total);
+          moved = 0;
+          for (size_t x = 0; x < total; ++x) moved += ops[i].present[x] || ops[i].goal == RSGPU_GOAL_ALL || x < c.k;
+        }
+        if (op == RSGPU_OP_VERIFY) b.any_verify = true;
+        B.algorithmic_bytes += uint64_t(moved) * ops[i].shard_len;
+      }
+      std::shared_ptr<LeoLaunch> L;
+      int rc = prepare_leo_sliced(c, op, lens.size(), sh.data(), pres.data(), lens.data(), std::get<2>(kv.first),
+                                  flag_of.data(), b.d_flags, s, b.stream_ordered, L);
+      if (rc) return rc;
+      b.side.push_back(L);
+      sliced_jobs += lens.size();
+    }
+  }
   uint8_t *base = static_cast<uint8_t *>(b.d_blob);
   const uint32_t *tbl_base = reinterpret_cast<const uint32_t *>(base + o_tbl);
   for (size_t ji = 0; ji < B.jobs.size(); ++ji) {
@@ -985,7 +1068,7 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
   a.n_items = uint32_t(items.size());
 
   b.info.n_ops = n_ops;
-  b.info.n_jobs = B.jobs.size();
+  b.info.n_jobs = B.jobs.size() + sliced_jobs;
   b.info.n_items = items.size();
   b.info.n_classes = B.classes.size();
   b.info.grid = uint32_t(b.grid);
@@ -1021,7 +1104,8 @@ int mix_launch(MixBatch &b, cudaStream_t s) {
     int rc = b.enqueue(s);
     if (rc) return rc;
   }
-  launch_counter_add(b.mix_kernels);  // the routed launches count themselves
+  // Launched one by one, the launches beside k_mix count themselves.
+  launch_counter_add(b.exec ? b.info.kernels_per_launch : b.mix_kernels);
   return RSGPU_OK;
 }
 

@@ -22,18 +22,36 @@ namespace {
 
 constexpr int kSliceMaxThreads = 1024;  // 64 registers
 
+// Work item x of a launch: its job, the tile's first column and the job's
+// shard length.
+struct SliceItem {
+  uint32_t job;
+  uint64_t tile, len;
+};
+template <int WT>
+__device__ __forceinline__ uint32_t slice_items(const SliceArgs &a) {
+  return a.items ? a.n_items : uint32_t((a.len + 32 * WT - 1) / (32 * WT)) * a.n_jobs;
+}
+template <int WT>
+__device__ __forceinline__ SliceItem slice_item(const SliceArgs &a, uint32_t x) {
+  if (a.items) {
+    const uint2 w = a.items[x];
+    return SliceItem{w.x, uint64_t(w.y) * (32 * WT), a.lens[w.x]};
+  }
+  const uint32_t tiles_per_job = uint32_t((a.len + 32 * WT - 1) / (32 * WT)), job = x / tiles_per_job;
+  return SliceItem{job, uint64_t(x - job * tiles_per_job) * (32 * WT), a.len};
+}
+
 template <int WT, bool VERIFY>
 __global__ void __launch_bounds__(kSliceMaxThreads, 1) k_slice_encode(SliceArgs a) {
   extern __shared__ __align__(16) uint4 slice_smem[];
-  constexpr uint64_t tile_bytes = 32 * WT;
-  const uint32_t tiles_per_job = uint32_t((a.len + tile_bytes - 1) / tile_bytes);
-  const uint32_t total = tiles_per_job * a.n_jobs;
+  const uint32_t total = slice_items<WT>(a);
 #pragma unroll 1
   for (uint32_t x = blockIdx.x; x < total; x += gridDim.x) {
-    const uint32_t job = x / tiles_per_job;
-    const uint64_t tile = uint64_t(x - job * tiles_per_job) * tile_bytes;
-    const LeoJob jd = a.jobs[job];
-    const uint32_t bad = slice_encode_tile<WT, VERIFY>(uint32_t(__cvta_generic_to_shared(slice_smem)), a, a.ptrs + jd.ptr_off, tile, a.len);
+    const SliceItem it = slice_item<WT>(a, x);
+    const LeoJob jd = a.jobs[it.job];
+    const uint32_t bad = slice_encode_tile<WT, VERIFY>(uint32_t(__cvta_generic_to_shared(slice_smem)), a,
+                                                       a.ptrs + jd.ptr_off, it.tile, it.len);
     if (VERIFY && __any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(a.flags + jd.flag_idx, 1u);
     __syncthreads();  // rows are free for the next tile
   }
@@ -45,20 +63,18 @@ __global__ void __launch_bounds__(kSliceMaxThreads, 1) k_slice_decode(SliceArgs 
   __shared__ __align__(8) uint8_t need_bits[8];
   uint64_t *lane_ptrs = reinterpret_cast<uint64_t *>(slice_smem + size_t(a.n) * 2 * WT);
   const LaneInfo info{lane_ptrs, reinterpret_cast<uint8_t *>(lane_ptrs + a.n)};
-  constexpr uint64_t tile_bytes = 32 * WT;
-  const uint32_t tiles_per_job = uint32_t((a.len + tile_bytes - 1) / tile_bytes);
-  const uint32_t total = tiles_per_job * a.n_jobs;
+  const uint32_t total = slice_items<WT>(a);
   uint32_t cur = ~0u;
 #pragma unroll 1
   for (uint32_t x = blockIdx.x; x < total; x += gridDim.x) {
-    const uint32_t job = x / tiles_per_job;
-    if (job != cur) {  // CTA-uniform; the rows and info are free (barrier below)
-      cur = job;
-      slice_lane_info(a, a.jobs[job], info, need_bits);
+    const SliceItem it = slice_item<WT>(a, x);
+    if (it.job != cur) {  // CTA-uniform; the rows and info are free (barrier below)
+      cur = it.job;
+      slice_lane_info(a, a.jobs[it.job], info, need_bits);
       __syncthreads();
     }
-    slice_decode_tile<WT>(uint32_t(__cvta_generic_to_shared(slice_smem)), a, info, need_bits, a.jobs[job].input_count,
-                          uint64_t(x - job * tiles_per_job) * tile_bytes, a.len);
+    slice_decode_tile<WT>(uint32_t(__cvta_generic_to_shared(slice_smem)), a, info, need_bits,
+                          a.jobs[it.job].input_count, it.tile, it.len);
     __syncthreads();
   }
 }
@@ -84,17 +100,32 @@ bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t columns) {
   return k <= 4 * m && (m == 16 || columns >= (2 << 20));
 }
 
-int slice_configure(int op, SliceArgs &a, SliceShape &sh) {
+namespace {
+// Rows, threads a row and shared memory of a tile.
+void slice_tile(int op, SliceArgs &a, SliceShape &sh) {
   constexpr size_t kLimit = 227 * 1024 - 256;  // a CTA's shared memory less the static part
   a.rows = slice_rows(op, a.k, a.m, a.n);
   const size_t info = op == RSGPU_OP_RECONSTRUCT ? size_t(a.n) * LaneInfo::kBytes : 0;
-  const uint32_t lanes = op == RSGPU_OP_RECONSTRUCT ? a.n : a.m;
-  const uint32_t items = std::max(1u, lanes / 4);  // radix-4 groups of a pass: one per warp
   a.wt = 32;
   // 28 threads a row when 256 rows would not fit at 32, and when it lets a
   // second CTA share the SM (128 rows).
   if (size_t(a.rows) * 32 * a.wt + info > kLimit || (a.rows == 128 && !info)) a.wt = 28;
   sh.smem = size_t(a.rows) * 32 * a.wt + info;
+}
+}  // namespace
+
+uint64_t slice_tile_bytes(int op, uint32_t k, uint32_t m, uint32_t n) {
+  SliceArgs a{};
+  SliceShape sh;
+  a.k = k, a.m = m, a.n = n;
+  slice_tile(op, a, sh);
+  return 32 * uint64_t(a.wt);
+}
+
+int slice_configure(int op, SliceArgs &a, SliceShape &sh) {
+  slice_tile(op, a, sh);
+  const uint32_t lanes = op == RSGPU_OP_RECONSTRUCT ? a.n : a.m;
+  const uint32_t items = std::max(1u, lanes / 4);  // radix-4 groups of a pass: one per warp
   const uint32_t ctas = std::max<uint32_t>(1, uint32_t(227 * 1024 / (sh.smem + 1280)));
   uint32_t warps = 1;
   while (warps * 2 <= items && warps * 2 * ctas <= 32 + 16) warps *= 2;
@@ -104,7 +135,7 @@ int slice_configure(int op, SliceArgs &a, SliceShape &sh) {
   int per_sm = 0;
   RS_CUDA(blocks_per_sm(fn, sh.threads, sh.smem, &per_sm));
   const uint64_t tile = uint64_t(32) * a.wt;
-  const uint64_t tiles = ((a.len + tile - 1) / tile) * std::max<uint32_t>(a.n_jobs, 1);
+  const uint64_t tiles = a.items ? a.n_items : ((a.len + tile - 1) / tile) * std::max<uint32_t>(a.n_jobs, 1);
   sh.grid = int(std::min<uint64_t>(tiles, uint64_t(std::max(per_sm, 1)) * device_sm_count()));
   return RSGPU_OK;
 }

@@ -32,6 +32,7 @@ bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t columns);
 // Fills the tile width and rows of `a` (its geometry, len and n_jobs set) and
 // the launch shape of operation op (RSGPU_OP_*).
 int slice_configure(int op, SliceArgs &a, SliceShape &sh);
+uint64_t slice_tile_bytes(int op, uint32_t k, uint32_t m, uint32_t n);
 int slice_launch(int op, const SliceArgs &a, const SliceShape &sh, cudaStream_t s);
 // Tower coordinates of the element of each log value of the 8- or 16-bit
 // field, from its exp table.

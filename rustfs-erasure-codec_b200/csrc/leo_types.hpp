@@ -57,6 +57,10 @@ struct SliceArgs {
   uint32_t k, p, m, n, mod;
   uint32_t wt;  // threads per row: a tile is 32 * wt bytes of every shard
   uint32_t rows;
+  // Jobs of different lengths: items[x] = (job, tile) and lens[job].
+  const uint2 *items;
+  const uint64_t *lens;
+  uint32_t n_items;
 };
 
 // Launch of the bit-sliced GF(2^16) transforms (slice16.cuh): one chunk of

@@ -922,9 +922,12 @@ int copy_locators(LeopardState &st, const std::vector<LeoPlan *> &plans, uint16_
   return RSGPU_OK;
 }
 
+// With `lens` (a length per stripe; GF(2^8), every pointer 16-byte aligned) the
+// launch runs the bit-sliced kernels over all of them; flag_of then gives each
+// stripe's verify flag.
 int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const uint8_t *present, size_t len,
               int goal, const uint8_t *required, size_t n_required, uint32_t *flags, LeoLaunch &L,
-              cudaStream_t s, bool one_shot) {
+              cudaStream_t s, bool one_shot, const size_t *lens = nullptr, const uint32_t *flag_of = nullptr) {
   LeopardState &st = *c.leo;
   const size_t total = c.k + c.m;
   L.codec = &c;
@@ -933,6 +936,9 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
   std::vector<LeoJob> jobs;
   std::vector<uint8_t> roles;
   std::vector<size_t> role_off;
+  std::vector<uint64_t> job_lens;  // with lens: per job, and the (job, tile) items
+  std::vector<uint2> items;
+  size_t o_lens = 0, o_items = 0;
   {
     // The lock covers the plans, their locator launches and the copies of the
     // locators into this launch's blob.
@@ -946,7 +952,7 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
     for (size_t i = 0; i < n_stripes && bad == RSGPU_OK; ++i) {
       LeoJob j{};
       j.ptr_off = uint32_t(i * total);
-      j.flag_idx = uint32_t(i);
+      j.flag_idx = flag_of ? flag_of[i] : uint32_t(i);
       if (L.decode) {
         const uint8_t *pr = present + i * total;
         size_t np = 0;
@@ -979,18 +985,29 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
         role_off.push_back(base);
       }
       jobs.push_back(j);
+      if (lens) job_lens.push_back(lens[i]);
     }
     int rc = build_locators(c, pending, s);  // plans already cached get their locators even on an error
     if (rc) return rc;
     if (bad) return bad;
-    // Blob: jobs | pointers | roles | locators (one array per distinct pattern).
+    if (lens) {
+      const uint64_t tile = slice_tile_bytes(op, uint32_t(c.k), st.m, st.n);
+      for (size_t j = 0; j < jobs.size(); ++j)
+        for (uint64_t t = 0; t * tile < job_lens[j]; ++t) items.push_back(make_uint2(uint32_t(j), uint32_t(t)));
+    }
+    // Blob: jobs | pointers | roles | lengths | items | locators (one array
+    // per distinct pattern).
     const size_t jb = jobs.size() * sizeof(LeoJob);
     const size_t pb = n_stripes * total * sizeof(void *);
-    const size_t lo = (jb + pb + roles.size() + 255) & ~size_t(255);
+    o_lens = (jb + pb + roles.size() + 15) & ~size_t(15);
+    o_items = o_lens + job_lens.size() * 8;
+    const size_t lo = (o_items + items.size() * sizeof(uint2) + 255) & ~size_t(255);
     const size_t lb = used.size() * size_t(st.n) * 2;
     std::vector<uint8_t> blob(lo);
     std::memcpy(blob.data() + jb, shards, pb);
     std::memcpy(blob.data() + jb + pb, roles.data(), roles.size());
+    std::memcpy(blob.data() + o_lens, job_lens.data(), job_lens.size() * 8);
+    std::memcpy(blob.data() + o_items, items.data(), items.size() * sizeof(uint2));
     if (one_shot) {
       RS_CUDA(cudaError_t(lib_malloc_async(&L.d_blob, lo + lb + 16, s)));
       L.blob_ordered = true;
@@ -1062,7 +1079,7 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
     }
   }
   if (L.engine == 1 && st.field->bits == 8) {
-    if ((low & 15) == 0 && slice_pays(op, a.k, a.m, a.n, uint64_t(len) * a.n_jobs)) {
+    if ((low & 15) == 0 && (lens || slice_pays(op, a.k, a.m, a.n, uint64_t(len) * a.n_jobs))) {
       L.engine = 2;
       SliceArgs &sa = L.slice;
       sa.jobs = a.jobs;
@@ -1076,9 +1093,15 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
       sa.m = a.m;
       sa.n = a.n;
       sa.mod = a.mod;
+      if (lens) {
+        sa.lens = reinterpret_cast<const uint64_t *>(dbase + o_lens);
+        sa.items = reinterpret_cast<const uint2 *>(dbase + o_items);
+        sa.n_items = uint32_t(items.size());
+      }
       return slice_configure(op, sa, L.slice_shape);
     }
   }
+  if (lens) return RSGPU_ERR_INVALID_ARGUMENT;
   if (L.engine == 1) {
     const bool b16f = st.field->bits == 16;
     const size_t nj = jobs.size();
@@ -1257,6 +1280,21 @@ int prepare_leo_reconstruct_once(Codec &c, size_t n, uint8_t *const *shards, con
   if (rc) return rc;
   out = L;
   return RSGPU_OK;
+}
+
+int prepare_leo_sliced(Codec &c, int op, size_t n, uint8_t *const *shards, const uint8_t *present, const size_t *lens,
+                       int goal, const uint32_t *flag_of, uint32_t *flags, cudaStream_t s, bool one_shot,
+                       std::shared_ptr<LeoLaunch> &out) {
+  auto L = std::make_shared<LeoLaunch>();
+  int rc = build_leo(c, op, n, shards, present, 0, goal, nullptr, 0, flags, *L, s, one_shot, lens, flag_of);
+  if (rc) return rc;
+  out = L;
+  return RSGPU_OK;
+}
+
+bool leo_slice_takes(Codec &c, int op, uint64_t columns) {
+  const LeopardState &st = *c.leo;
+  return st.field->bits == 8 && leo_engine() == 1 && slice_pays(op, uint32_t(c.k), st.m, st.n, columns);
 }
 
 static int run_once(Codec &c, int op, size_t n, uint8_t *const *shards, const uint8_t *present, size_t len, int goal,

@@ -35,6 +35,15 @@ int leo_launch(const LeoLaunch &l, cudaStream_t s);
 int prepare_leo_reconstruct_once(Codec &c, size_t n, uint8_t *const *shards, const uint8_t *present, size_t len,
                                  int goal, cudaStream_t s, void *scratch, std::shared_ptr<LeoLaunch> &out);
 size_t leo_reconstruct_scratch_bytes(Codec &c);
+// One launch of the bit-sliced GF(2^8) kernels over n stripes of one codec and
+// operation with a length each (16-byte-aligned shards; flag_of: each stripe's
+// verify flag in `flags`).  one_shot: built on stream s without waiting, its
+// memory freed there behind the kernel.
+int prepare_leo_sliced(Codec &c, int op, size_t n, uint8_t *const *shards, const uint8_t *present, const size_t *lens,
+                       int goal, const uint32_t *flag_of, uint32_t *flags, cudaStream_t s, bool one_shot,
+                       std::shared_ptr<LeoLaunch> &out);
+// Whether those kernels are the faster ones for this much work in all.
+bool leo_slice_takes(Codec &c, int op, uint64_t columns);
 void leo_set_scratch(LeoLaunch &l, void *scratch);
 int prepare_tower(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const uint8_t *present, size_t len,
                   int goal, uint32_t *flags, std::shared_ptr<LeoLaunch> &out);
