@@ -354,9 +354,70 @@ __device__ __forceinline__ void slice_lane_info(const SliceArgs &a, const LeoJob
   }
 }
 
+// The middle of a decode over n = 2^b lanes, b >= 4, in place: the two highest
+// IFFT layers, the formal derivative (src/core/leopard_gf16/decode.rs:
+// 1100-1116: lane l gains the lanes l | 2^t over its zero bits t) and the two
+// highest FFT layers, on lanes a, a + n/4, a + n/2, a + 3n/4.  With V the rows
+// before, W = IFFT_top(V) and N_low, N_top the derivative's parts over the low
+// bits and the top two,
+//   FFT_top(W + N_top W + N_low W) = FFT_top((1 + N_top) IFFT_top V) + N_low V,
+// because the FFT undoes the IFFT and acts on every a alike.  The block is the
+// transform's first, so all its constants are fixed.  A row depends on rows of
+// the same or a larger a, so with a taken in ascending rounds each round reads
+// everything, waits for the CTA, then writes.
+template <int WT>
+__device__ __forceinline__ void slice_middle(const Rows<WT> &s, uint32_t n) {
+  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, items = n >> 2;
+  const uint32_t quarter = items * Rows<WT>::kStride;
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < items; i0 += warps) {
+    const uint32_t a = min(i0 + warp, items - 1);  // past the last: redone, not stored
+    const uint32_t base = s.at(a);
+    uint32_t v[4][8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) Rows<WT>::load(base + j * quarter, v[j]);
+    xor_planes<8>(v[1], v[0]);  // IFFT_top
+    xor_planes<8>(v[3], v[2]);
+    mac_const<8, 2>(v[2], v[3]);
+    xor_planes<8>(v[2], v[0]);
+    xor_planes<8>(v[3], v[1]);
+    xor_planes<8>(v[0], v[1]);  // 1 + N_top
+    xor_planes<8>(v[0], v[2]);
+    xor_planes<8>(v[1], v[3]);
+    xor_planes<8>(v[2], v[3]);
+    xor_planes<8>(v[2], v[0]);  // FFT_top
+    xor_planes<8>(v[3], v[1]);
+    mac_const<8, 2>(v[2], v[3]);
+    xor_planes<8>(v[1], v[0]);
+    xor_planes<8>(v[3], v[2]);
+#pragma unroll 1
+    for (uint32_t t = 1; t < items; t <<= 1) {
+      if (a & t) continue;  // warp-uniform
+      const uint32_t src = base + t * Rows<WT>::kStride;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t u[8];
+        Rows<WT>::load(src + j * quarter, u);
+        xor_planes<8>(v[j], u);
+      }
+    }
+    __syncthreads();
+    if (i0 + warp < items) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s.store(base + j * quarter, v[j]);
+    }
+    __syncthreads();
+  }
+}
+
 // Reconstruct one tile: present lanes scaled by their locators, IFFT, formal
 // derivative, FFT, targets scaled by the inverse locators.  info holds the
-// job's lanes and need the 4-lane blocks that hold a target.
+// job's lanes and need the 4-lane blocks that hold a target.  From 16 lanes on
+// the first two layers take their lanes straight from the shards (four shards'
+// loads in flight), the middle is one pass and the last two layers give theirs
+// straight to the targets: 128+64 at 512 KiB x 16, 32 lost, 2218 -> 1950 us.
+// The encode keeps a load and a store pass of its own: fused the same way, its
+// small CTAs waited for instructions (32+16 encode 663 -> 693 us).
 template <int WT>
 __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs &a, LaneInfo info, const uint8_t *need,
                                                   uint32_t input_count, uint64_t tile, uint64_t len) {
@@ -364,6 +425,95 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
   const uint32_t n = a.n, b = 31 - __clz(n);
   const Rows<WT> s(smem, t);
   const Cols<WT> cols(tile, t, len);
+  if (b >= 4) {
+#pragma unroll 1
+    for (uint32_t q = warp; q < (n >> 2); q += warps) {
+      const uint32_t r = 4 * q;
+      uint32_t v[4][8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[j][i] = 0;
+        const uint64_t ptr = info.ptr[r + j];
+        if (ptr & 1) cols.load(reinterpret_cast<const uint8_t *>(ptr - 1), v[j]);  // warp-uniform
+      }
+      if (r < input_count) {
+        // Four rounds over one copy of the networks, the lanes rotating
+        // through v[0].
+#pragma unroll 1
+        for (uint32_t j = 0; j < 4; ++j) {
+          uint32_t x[8] = {};
+          if (info.ptr[r + j] & 1) {  // warp-uniform
+            slice8(v[0]);
+            planes_to_tower<8>(v[0]);
+            mac<8>(info.c[r + j], x, v[0]);
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            v[0][i] = v[1][i];
+            v[1][i] = v[2][i];
+            v[2][i] = v[3][i];
+            v[3][i] = x[i];
+          }
+        }
+        ifft4(v, tower_const<8>(r), tower_const<8>(r >> 1));
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s.store(s.at(r + j), v[j]);
+    }
+    __syncthreads();
+    // Layers 2 .. b - 3: for an odd b the first of them alone.
+    uint32_t lgd = 2;
+    if (b & 1) {
+      slice_pass2<WT, false>(s, s, false, n, lgd++, 0);
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (; lgd < b - 2; lgd += 2) {
+      slice_pass4<WT, false>(s, s, false, n, lgd, 0, input_count, ~0ull);
+      __syncthreads();
+    }
+    slice_middle<WT>(s, n);
+    const uint64_t blocks = *reinterpret_cast<const uint64_t *>(need);
+    const uint32_t limit = a.m + a.k;
+#pragma unroll 1
+    while (lgd > 2 + (b & 1)) {
+      lgd -= 2;
+      slice_pass4<WT, true>(s, s, false, n, lgd, 0, limit, blocks);
+      __syncthreads();
+    }
+    if (b & 1) {
+      slice_pass2<WT, true>(s, s, false, n, 2, 0);
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (uint32_t q = warp; q < (n >> 2); q += warps) {
+      const uint32_t r = 4 * q;
+      if (!((blocks >> q) & 1)) continue;  // warp-uniform
+      uint32_t v[4][8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Rows<WT>::load(s.at(r + j), v[j]);
+      fft4(v, tower_const<8>(r), tower_const<8>(r >> 1));
+#pragma unroll 1
+      for (uint32_t j = 0; j < 4; ++j) {
+        const uint64_t ptr = info.ptr[r + j];
+        if (ptr & 2) {  // warp-uniform
+          uint32_t x[8] = {};
+          mac<8>(info.c[r + j], x, v[0]);
+          planes_to_cantor<8>(x);
+          slice8(x);
+          cols.store(reinterpret_cast<uint8_t *>(ptr - 2), x);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[0][i] = v[1][i];
+          v[1][i] = v[2][i];
+          v[2][i] = v[3][i];
+        }
+      }
+    }
+    return;
+  }
 #pragma unroll 1
   for (uint32_t i = warp; i < n; i += warps) {
     uint32_t x[8] = {};
