@@ -6,16 +6,11 @@
 // (or 32) byte columns of one stripe and reads every input shard exactly once
 // with coalesced 128-bit loads.  Products are table lookups split over the
 // bits of the data byte, and the tables of four outputs are packed into one
-// 32-bit word per entry, so one lookup serves four output rows.  Two
-// formulations can share the work so that neither the shuffle (LSU) pipe nor
-// the integer (ALU) pipe saturates:
-//   4+4 split: two warp-shuffle lookups into 16-entry tables held one entry
-//     per lane (mirrored into lanes 16..31, so the raw shifted data word is a
-//     valid index: the shuffle only reads bits 0..4);
-//   5+3 split: one shuffle into a 32-entry table for the low five bits and one
-//     byte-permute (PRMT) per output for the high three bits, whose eight-entry
-//     byte table fits the two PRMT source registers and whose result lands
-//     directly in per-output column order.
+// 32-bit word per entry, so one lookup serves four output rows.  A lookup is a
+// warp shuffle into a 32-entry table held one entry per lane; how bytes share
+// lookups is described at Lut below.  The staged tile of k_classic.cu uses
+// pairs of 16-entry tables instead (4+4 split; a table mirrored into lanes
+// 16..31 makes the raw shifted data word a valid index).
 // All outputs of a column are accumulated in registers and written once.
 // The tables need not come from the classic field: any GF(2)-linear byte map
 // (multiplication by a constant in the Leopard GF(2^8) field, for one) packs
@@ -55,14 +50,6 @@ __device__ __forceinline__ void transpose4(const uint32_t *a, uint32_t *o) {
   o[1] = __byte_perm(t0, t1, 0x7632);
   o[2] = __byte_perm(t2, t3, 0x5410);
   o[3] = __byte_perm(t2, t3, 0x7632);
-}
-
-// 5+3 split, shuffle half: low five bits of each byte of w index t5.
-__device__ __forceinline__ void mac4_lo5(uint32_t w, uint32_t t5, uint32_t *a) {
-  a[0] ^= tshfl(t5, w);
-  a[1] ^= tshfl(t5, w >> 8);
-  a[2] ^= tshfl(t5, w >> 16);
-  a[3] ^= tshfl(t5, w >> 24);
 }
 
 // 5+3 split, PRMT half: selector nibble c = high three bits of byte c of w.
@@ -193,14 +180,48 @@ struct LutSet {
   }
 };
 
+// Inputs j0 .. j0 + C of one tile and pass: loads, tables and products.
+template <int C, int NG, int V>
+__device__ __forceinline__ void apply_step(const uint8_t *const *ptr, const JobDesc &d, uint32_t g0, uint32_t groups,
+                                           uint32_t j0, const uint64_t *col, const bool *active, uint32_t lane,
+                                           uint32_t (*acc)[V][16]) {
+  uint4 x[C][V];
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    const uint8_t *src = ptr[j0 + i];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      x[i][v] = make_uint4(0, 0, 0, 0);
+      if (active[v]) x[i][v] = ld_stream(src + col[v]);
+    }
+  }
+  Lut<C> lut[NG];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    const uint32_t *tbl = d.tbl + (size_t(g0 + (uint32_t(g) < groups ? g : 0)) * d.n_in + j0) * kTableWords;
+    lut_load<C>(lut[g], lane, [&](int i, uint32_t w) { return __ldg(tbl + i * kTableWords + w); });
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      uint32_t y[C], m[Lut<C>::kMixed];
+#pragma unroll
+      for (int i = 0; i < C; ++i) y[i] = w == 0 ? x[i][v].x : w == 1 ? x[i][v].y : w == 2 ? x[i][v].z : x[i][v].w;
+      lut_index<C>(y, m);
+#pragma unroll
+      for (int g = 0; g < NG; ++g)
+        if (g == 0 || uint32_t(g) < groups) lut_mac<C>(lut[g], y, m, &acc[g][v][4 * w]);  // CTA-uniform
+    }
+}
+
 // One tile = kApplyThreads threads x V 128-bit vectors of columns of job d,
 // starting at byte tile_base (< d.vec_len).  NG = number of 4-output groups
-// per pass over the inputs (outputs g*4 .. g*4+3).  MIX: 0 = every input uses
-// the 4+4 split, 1 = odd inputs use 5+3, 2 = all 5+3.  Must be called by all
+// per pass over the inputs (outputs g*4 .. g*4+3).  Must be called by all
 // kApplyThreads threads of the CTA (warp shuffles need full warps).
 // ACC: outputs accumulate (dst ^= product) instead of being overwritten,
 // for incremental parity updates (encode_single with i > 0, update).
-template <int NG, int V, int kBatch, int MIX, bool VERIFY, bool ACC = false>
+template <int NG, int V, bool VERIFY, bool ACC = false>
 __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t *flags, const JobDesc &d,
                                            uint64_t tile_base) {
   const uint32_t lane = threadIdx.x & 31;
@@ -216,62 +237,23 @@ __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t 
   const uint8_t *const *ptr = ptrs + d.ptr_off;
   const uint32_t n_in = d.n_in;
   for (uint32_t g0 = 0; g0 * 4 < d.n_out; g0 += NG) {
-    uint32_t acc[NG][V][16];   // per column: 4 packed outputs
-    uint32_t oacc[NG][V][16];  // per output r, word w (index r*4+w): 4 columns
+    const uint32_t groups = min(uint32_t(NG), (d.n_out + 3) / 4 - g0);
+    uint32_t acc[NG][V][16];  // per column: 4 packed outputs
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
       for (int v = 0; v < V; ++v)
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[g][v][i] = oacc[g][v][i] = 0;
-    for (uint32_t j0 = 0; j0 < n_in; j0 += kBatch) {
-      uint4 x[kBatch][V];
-#pragma unroll
-      for (int b = 0; b < kBatch; ++b) {
-        const uint8_t *src = (j0 + b < n_in) ? ptr[j0 + b] : nullptr;
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          x[b][v] = make_uint4(0, 0, 0, 0);
-          if (src && active[v]) x[b][v] = ld_stream(src + col[v]);
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < kBatch; ++b) {
-        if (j0 + b >= n_in) break;  // warp-uniform
-        const bool split53 = MIX == 2 || (MIX == 1 && (b & 1));  // compile-time
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-          const uint32_t *tb = d.tbl + ((g0 + g) * n_in + (j0 + b)) * kTableWords;
-          if (!split53) {
-            const uint32_t lo = __ldg(tb + (lane & 15));
-            const uint32_t hi = __ldg(tb + 16 + (lane & 15));
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-              mac4(x[b][v].x, lo, hi, &acc[g][v][0]);
-              mac4(x[b][v].y, lo, hi, &acc[g][v][4]);
-              mac4(x[b][v].z, lo, hi, &acc[g][v][8]);
-              mac4(x[b][v].w, lo, hi, &acc[g][v][12]);
-            }
-          } else {
-            const uint32_t t5 = __ldg(tb + 32 + lane);
-            const uint4 h01 = __ldg(reinterpret_cast<const uint4 *>(tb + 64));
-            const uint4 h23 = __ldg(reinterpret_cast<const uint4 *>(tb + 68));
-            const uint32_t h3[8] = {h01.x, h01.y, h01.z, h01.w, h23.x, h23.y, h23.z, h23.w};
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-              const uint32_t wv[4] = {x[b][v].x, x[b][v].y, x[b][v].z, x[b][v].w};
-#pragma unroll
-              for (int w = 0; w < 4; ++w) {
-                mac4_lo5(wv[w], t5, &acc[g][v][w * 4]);
-                const uint32_t sel = hi3_selector(wv[w]);
-#pragma unroll
-                for (int r = 0; r < 4; ++r) oacc[g][v][r * 4 + w] ^= __byte_perm(h3[2 * r], h3[2 * r + 1], sel);
-              }
-            }
-          }
-        }
-      }
+        for (int i = 0; i < 16; ++i) acc[g][v][i] = 0;
+    uint32_t j = 0;
+#pragma unroll 1
+    for (; j + 5 <= n_in; j += 5) apply_step<5, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
+    if (j + 3 <= n_in) {
+      apply_step<3, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
+      j += 3;
     }
+#pragma unroll 1
+    for (; j < n_in; ++j) apply_step<1, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
     bool bad = false;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
@@ -283,7 +265,7 @@ __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t 
           uint32_t tmp[4];
           transpose4(&acc[g][v][w * 4], tmp);
 #pragma unroll
-          for (int r = 0; r < 4; ++r) o[r][w] = tmp[r] ^ (MIX ? oacc[g][v][r * 4 + w] : 0u);
+          for (int r = 0; r < 4; ++r) o[r][w] = tmp[r];
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {

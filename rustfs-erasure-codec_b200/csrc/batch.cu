@@ -144,13 +144,15 @@ __global__ void __launch_bounds__(kMixThreads, kMixBlocks) k_mix(MixArgs a) {
         if (bad) atomicOr(a.flags + d.flag_idx, 1u);
       } else {
         const uint64_t t = item.tile;
-        switch (kind) {
-          case 0: apply_tile<1, 2, 4, 0, false>(a.ptrs, a.flags, d, t * (2 * kApplyTile)); break;
-          case 1: apply_tile<1, 1, 4, 0, false>(a.ptrs, a.flags, d, t * kApplyTile); break;
-          case 2: apply_tile<2, 1, 4, 0, false>(a.ptrs, a.flags, d, t * kApplyTile); break;
-          case 4: apply_tile<1, 2, 4, 0, true>(a.ptrs, a.flags, d, t * (2 * kApplyTile)); break;
-          case 5: apply_tile<1, 1, 4, 0, true>(a.ptrs, a.flags, d, t * kApplyTile); break;
-          default: apply_tile<2, 1, 4, 0, true>(a.ptrs, a.flags, d, t * kApplyTile); break;
+        // Kind 0 is two tiles of 4 KiB.  One tile shape for every kind: its 16
+        // sums fit the kernel's registers, which 8 outputs a pass or 32 bytes a
+        // thread did not (spill loads 5.6 -> 4.0 KB).
+        const uint64_t first = (kind & 3) ? t : 2 * t, end = (kind & 3) ? t + 1 : 2 * t + 2;
+        for (uint64_t x = first; x < end && x * kApplyTile < d.vec_len; ++x) {
+          if (kind & MK_APPLY_VERIFY)
+            apply_tile<1, 1, true>(a.ptrs, a.flags, d, x * kApplyTile);
+          else
+            apply_tile<1, 1, false>(a.ptrs, a.flags, d, x * kApplyTile);
         }
       }
     } else {
@@ -437,23 +439,33 @@ cudaError_t grow_slot(ScratchSlot &slot, size_t need, cudaStream_t s) {
 // Only the order of the queue depends on it; the cost model refines it.
 double item_cost(uint64_t tile_bytes, size_t shards, double factor) { return double(tile_bytes) * shards * factor; }
 
-int add_apply_job(MixBuild &B, const rsgpu_plan &plan, bool verify, size_t n_in, size_t n_out, size_t ptr_off,
-                  size_t len, uint32_t flag_idx, const uint32_t *dev_tbl, size_t host_tbl) {
+// A K1 operation as jobs of at most 4 outputs (one pass over the inputs each):
+// the kernel would make those passes anyway, and as jobs of their own they are
+// work items a fraction as long.  A 128+64 rebuild of 16 shards was items of
+// ~370 us, and a batch waited for the last of them.
+void add_apply_job(MixBuild &B, const rsgpu_plan &plan, bool verify, size_t n_in, size_t n_out, size_t ptr_off,
+                   size_t len, uint32_t flag_idx, const uint32_t *dev_tbl, size_t host_tbl) {
   const uint32_t kind = uint32_t(plan.tile) | (verify ? MK_APPLY_VERIFY : 0u);
-  MixJob j{};
-  j.cls = B.apply_cls(kind);
-  j.len = len;
-  j.d.ptr_off = uint32_t(ptr_off);
-  j.d.n_in = uint16_t(n_in);
-  j.d.n_out = uint16_t(n_out);
-  j.d.flag_idx = flag_idx;
-  j.d.tbl = dev_tbl;
   bool aligned = true;
   for (size_t i = 0; i < n_in + n_out; ++i) aligned &= (reinterpret_cast<uintptr_t>(B.ptrs[ptr_off + i]) & 15) == 0;
-  j.d.vec_len = aligned ? (len & ~uint64_t(15)) : 0;
-  const double passes = double((n_out + 3) / 4);
-  B.push_job(j, host_tbl, item_cost(1, n_in + n_out, 1.0 + 0.1 * passes * n_in / 16.0));
-  return RSGPU_OK;
+  for (size_t o = 0; o < n_out; o += 4) {
+    const size_t outs = std::min<size_t>(4, n_out - o), tbl = o / 4 * n_in * kTableWords;
+    MixJob j{};
+    j.cls = B.apply_cls(kind);
+    j.len = len;
+    j.d.ptr_off = uint32_t(ptr_off);
+    if (o) {
+      j.d.ptr_off = uint32_t(B.ptrs.size());
+      for (size_t i = 0; i < n_in; ++i) B.ptrs.push_back(B.ptrs[ptr_off + i]);
+      for (size_t i = 0; i < outs; ++i) B.ptrs.push_back(B.ptrs[ptr_off + n_in + o + i]);
+    }
+    j.d.n_in = uint16_t(n_in);
+    j.d.n_out = uint16_t(outs);
+    j.d.flag_idx = flag_idx;
+    j.d.tbl = dev_tbl ? dev_tbl + tbl : nullptr;
+    j.d.vec_len = aligned ? (len & ~uint64_t(15)) : 0;
+    B.push_job(j, host_tbl == SIZE_MAX ? SIZE_MAX : host_tbl + tbl, item_cost(1, n_in + outs, 1.0 + 0.1 * n_in / 16.0));
+  }
 }
 
 }  // namespace
@@ -528,13 +540,14 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
     }
   // Leopard GF(2^8) operations that the bit-sliced kernels run faster go in
   // one launch per (codec, operation, goal) beside k_mix (planners TABLE and
-  // MODEL; the fixed rule and forced plans stay in k_mix).  Encodes and
-  // verifies always; rebuilds unless the dense map in k_mix takes less: its
-  // time goes with present * ceil(targets / 4), theirs with lanes * layers.
+  // MODEL; the fixed rule and forced plans stay in k_mix).  Encodes, verifies
+  // and rebuilds planned as transforms always; rebuilds planned as dense maps
+  // unless the map in k_mix takes less: its time goes with present *
+  // ceil(targets / 4), theirs with lanes * layers.
   // One B200, 8 stripes of 512 KiB shards, dense map / bit-sliced, us:
-  //   rebuild 128+64, 4 lost 314 / 1013, 16 lost 867 / 1082, 24 lost 1232 / 1098, 64 lost 2486 / 1142
-  //   rebuild 32+16, 4 lost 83 / 202, 16 lost 169 / 216;  60+20, 16 lost 322 / 521
-  //   encode 128+64 2419 (FFT in k_mix 984) / 487, 32+16 182 / 91, 20+8 61 / 55
+  //   rebuild 128+64, 4 lost 255 / 908, 16 lost 792 / 968, 24 lost 1127 / 973, 64 lost 2273 / 1002
+  //   rebuild 32+16, 4 lost 65 / 178, 16 lost 161 / 187;  60+20, 16 lost 322 / 521
+  //   encode 128+64 2259 (FFT in k_mix 984) / 488, 32+16 175 / 89, 20+8 61 / 55
   std::vector<char> sliced(n_ops, 0);
   if (!forced && opt.planner != RSGPU_PLANNER_FIXED) {
     constexpr uint64_t kSlicedMinColumns = 256 << 10;  // below, a launch of its own does not pay
@@ -557,7 +570,9 @@ int mix_build(const rsgpu_mix_op *ops, size_t n_ops, const rsgpu_plan *forced, c
         if (low & 15) continue;
         if (ops[i].op == RSGPU_OP_RECONSTRUCT) {
           while ((1u << layers) < g.n) ++layers;
-          if (!targets || present * ((targets + 3) / 4) * 22 <= g.n * layers * 10) continue;
+          if (!targets || (b.plans[i].algo == RSGPU_ALGO_APPLY &&
+                           present * ((targets + 3) / 4) * 22 <= g.n * layers * 10))
+            continue;
         }
         uint64_t &sum = columns[std::make_tuple(&ops[i].codec->c, int(ops[i].op))];
         if (pass == 0)

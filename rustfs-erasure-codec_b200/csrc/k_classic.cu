@@ -27,8 +27,8 @@ namespace {
 // Grid-stride loop of apply_tile over every (job, tile) of a launch, inputs
 // loaded straight into registers: the tile for more than 4 outputs and for
 // accumulating (incremental parity) launches.
-template <int NG, int V, int kBatch, int MIX, bool VERIFY, bool ACC = false>
-__global__ void __launch_bounds__(kApplyThreads, (NG == 1 && V <= 2) ? 4 : 1) k_apply_vec(ApplyArgs a) {
+template <int NG, int V, bool VERIFY, bool ACC, int MINB>
+__global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(ApplyArgs a) {
   constexpr uint32_t kTile = kApplyThreads * kApplyVec * V;
   const uint32_t tiles_per_job = uint32_t((a.len + kTile - 1) / kTile);
   const uint32_t total = tiles_per_job * a.n_jobs;
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kApplyThreads, (NG == 1 && V <= 2) ? 4 : 1) k_
     const uint64_t tile_base = uint64_t(t - job * tiles_per_job) * kTile;
     const JobDesc d = a.jobs[job];
     if (tile_base >= d.vec_len) continue;  // CTA-uniform
-    apply_tile<NG, V, kBatch, MIX, VERIFY, ACC>(a.ptrs, a.flags, d, tile_base);
+    apply_tile<NG, V, VERIFY, ACC>(a.ptrs, a.flags, d, tile_base);
   }
 }
 
@@ -780,14 +780,15 @@ int grid_for(const void *fn, int threads, size_t smem) {
   return sms * per_sm;
 }
 
-template <int NG, int V, int B, int MIX, bool VERIFY, bool ACC = false>
+template <int NG, int V, bool VERIFY, bool ACC, int MINB>
 void launch_vec(const ApplyArgs &a, cudaStream_t s) {
   static int grid_max = 0;
-  if (!grid_max) grid_max = grid_for((const void *)k_apply_vec<NG, V, B, MIX, VERIFY, ACC>, kApplyThreads, 0);
+  const void *fn = (const void *)k_apply_vec<NG, V, VERIFY, ACC, MINB>;
+  if (!grid_max) grid_max = grid_for(fn, kApplyThreads, 0);
   const uint64_t tile = uint64_t(kApplyThreads) * kApplyVec * V;
   const uint64_t tiles = ((a.len + tile - 1) / tile) * a.n_jobs;
   const int grid = int(tiles < uint64_t(grid_max) ? tiles : grid_max);
-  k_apply_vec<NG, V, B, MIX, VERIFY, ACC><<<grid, kApplyThreads, 0, s>>>(a);
+  k_apply_vec<NG, V, VERIFY, ACC, MINB><<<grid, kApplyThreads, 0, s>>>(a);
 }
 
 template <int V, int S, bool VERIFY>
@@ -836,7 +837,10 @@ void launch_unaligned(const ApplyArgs &a, cudaStream_t s) {
   k_apply_unaligned<VERIFY, ACC><<<grid, kApplyThreads + 32, 0, s>>>(a);
 }
 
-// More than 4 outputs: the register-path tile, 8 outputs a pass.  At most 4:
+// More than 4 outputs: the register-path tile, 8 outputs a pass at 128
+// registers (80 registers, three CTAs an SM, spill: 50+20 256 KiB x 32 807
+// against 1111 GB/s; one group a pass at 64 registers 1011, three 1066; with
+// 4+4 and 5+3 lookups an input, before the shared ones, 672).  At most 4:
 // tables in registers up to kRegInputs inputs a job (beyond, they no longer
 // fit), the staged tile with tables read per step for wider jobs and for
 // launches whose jobs differ in width.  One B200, GB/s, staged tile / tables
@@ -849,9 +853,9 @@ void launch_unaligned(const ApplyArgs &a, cudaStream_t s) {
 template <bool VERIFY>
 void launch_write_or_verify(const ApplyArgs &a, int variant, cudaStream_t s) {
   if (a.max_out > 4)
-    launch_vec<2, 1, 4, 1, VERIFY>(a, s);
+    launch_vec<2, 1, VERIFY, false, 2>(a, s);
   else if (variant == 1)
-    launch_vec<1, 2, 4, 0, VERIFY>(a, s);
+    launch_vec<1, 1, VERIFY, false, 4>(a, s);
   else if (variant == 0 && a.uni_in >= 1 && a.uni_in <= kRegInputs)
     launch_reg_k<VERIFY>(a, s);
   else
@@ -873,7 +877,7 @@ cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cud
   uint64_t launches = 0;
   if (a.any_vec && a.len >= 16) {
     if (a.accumulate)
-      launch_vec<1, 2, 4, 0, false, true>(a, s);
+      launch_vec<1, 1, false, true, 4>(a, s);
     else if (verify)
       launch_write_or_verify<true>(a, apply_variant(), s);
     else
