@@ -469,20 +469,6 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
     max_out = std::max<uint32_t>(max_out, j.n_out);
     any_vec |= j.vec_len > 0;
   }
-  const size_t jb = jobs.size() * sizeof(JobDesc);
-  std::vector<uint8_t> blob(jb + ptrs.size() * sizeof(void *));
-  std::memcpy(blob.data(), jobs.data(), jb);
-  std::memcpy(blob.data() + jb, ptrs.data(), ptrs.size() * sizeof(void *));
-  owned = persistent;
-  if (persistent) {
-    RS_CUDA(cudaMalloc(&d_blob, std::max<size_t>(blob.size(), 16)));
-    RS_CUDA(cudaMemcpy(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice));
-  } else {
-    int rc = upload(blob.data(), blob.size(), &d_blob, s);
-    if (rc) return rc;
-  }
-  args.jobs = static_cast<const JobDesc *>(d_blob);
-  args.ptrs = reinterpret_cast<const uint8_t *const *>(static_cast<char *>(d_blob) + jb);
   args.flags = flags;
   args.len = len;
   args.n_jobs = uint32_t(jobs.size());
@@ -492,6 +478,25 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   args.any_unaligned = any_unaligned;
   args.tbl_stage = tbl_stage;
   args.accumulate = accumulate ? 1 : 0;
+  owned = persistent;
+  if (!persistent && jobs.size() == 1 && ptrs.size() <= kInlinePtrs) {
+    args.job = jobs[0];
+    std::copy(ptrs.begin(), ptrs.end(), args.job_ptrs);
+    return RSGPU_OK;
+  }
+  const size_t jb = jobs.size() * sizeof(JobDesc);
+  std::vector<uint8_t> blob(jb + ptrs.size() * sizeof(void *));
+  std::memcpy(blob.data(), jobs.data(), jb);
+  std::memcpy(blob.data() + jb, ptrs.data(), ptrs.size() * sizeof(void *));
+  if (persistent) {
+    RS_CUDA(cudaMalloc(&d_blob, std::max<size_t>(blob.size(), 16)));
+    RS_CUDA(cudaMemcpy(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+  } else {
+    int rc = upload(blob.data(), blob.size(), &d_blob, s);
+    if (rc) return rc;
+  }
+  args.jobs = static_cast<const JobDesc *>(d_blob);
+  args.ptrs = reinterpret_cast<const uint8_t *const *>(static_cast<char *>(d_blob) + jb);
   return RSGPU_OK;
 }
 

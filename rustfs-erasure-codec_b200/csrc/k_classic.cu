@@ -24,20 +24,27 @@ namespace rsgpu {
 
 namespace {
 
+// The launch's jobs and pointer table; the arguments must be __grid_constant__,
+// so that their address can be taken.
+__device__ __forceinline__ const JobDesc *job_list(const ApplyArgs &a) { return a.jobs ? a.jobs : &a.job; }
+__device__ __forceinline__ const uint8_t *const *ptr_list(const ApplyArgs &a) { return a.jobs ? a.ptrs : a.job_ptrs; }
+
 // Grid-stride loop of apply_tile over every (job, tile) of a launch, inputs
 // loaded straight into registers: the tile for more than 4 outputs and for
 // accumulating (incremental parity) launches.
 template <int NG, int V, bool VERIFY, bool ACC, int MINB>
-__global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(ApplyArgs a) {
+__global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(const __grid_constant__ ApplyArgs a) {
+  const JobDesc *const jobs = job_list(a);
+  const uint8_t *const *const ptrs = ptr_list(a);
   constexpr uint32_t kTile = kApplyThreads * kApplyVec * V;
   const uint32_t tiles_per_job = uint32_t((a.len + kTile - 1) / kTile);
   const uint32_t total = tiles_per_job * a.n_jobs;
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const uint32_t job = t / tiles_per_job;
     const uint64_t tile_base = uint64_t(t - job * tiles_per_job) * kTile;
-    const JobDesc d = a.jobs[job];
+    const JobDesc d = jobs[job];
     if (tile_base >= d.vec_len) continue;  // CTA-uniform
-    apply_tile<NG, V, VERIFY, ACC>(a.ptrs, a.flags, d, tile_base);
+    apply_tile<NG, V, VERIFY, ACC>(ptrs, a.flags, d, tile_base);
   }
 }
 
@@ -102,7 +109,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 }
 
 template <int V, int S, bool VERIFY>
-__global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a) {
+__global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(const __grid_constant__ ApplyArgs a) {
+  const JobDesc *const jobs = job_list(a);
+  const uint8_t *const *const ptrs = ptr_list(a);
   constexpr uint32_t kSlot = kApplyThreads * kApplyVec * V;  // one input's slice of a tile
   extern __shared__ __align__(128) uint8_t tma_smem[];
   __shared__ __align__(8) uint64_t full[S], empty[S];
@@ -136,10 +145,10 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a
     for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const uint32_t job = t / tiles_per_job;
       const uint64_t base = uint64_t(t - job * tiles_per_job) * kSlot;
-      const JobDesc d = a.jobs[job];
+      const JobDesc d = jobs[job];
       if (base >= d.vec_len) continue;
       const uint32_t valid = uint32_t(d.vec_len - base < kSlot ? d.vec_len - base : kSlot);
-      const uint8_t *const *ptr = a.ptrs + d.ptr_off;
+      const uint8_t *const *ptr = ptrs + d.ptr_off;
       const bool tbl_copy = a.tbl_stage && d.tbl && (reinterpret_cast<uintptr_t>(d.tbl) & 15) == 0;
       const uint32_t steps = (d.n_in + 3) / 4 + (VERIFY ? 1 : 0);
       for (uint32_t step = 0; step < steps; ++step, ++it) {
@@ -177,7 +186,7 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const uint32_t job = t / tiles_per_job;
     const uint64_t base = uint64_t(t - job * tiles_per_job) * kSlot;
-    const JobDesc d = a.jobs[job];
+    const JobDesc d = jobs[job];
     if (base >= d.vec_len) continue;
     const uint32_t n_in = d.n_in;
     const bool tbl_copy = a.tbl_stage && d.tbl && (reinterpret_cast<uintptr_t>(d.tbl) & 15) == 0;  // as the producer decides
@@ -246,10 +255,10 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(ApplyArgs a
                 const uint4 e = lds128(slot0 + r * kSlot + v * kApplyThreads * kApplyVec);
                 bad |= (e.x != o[r][0]) | (e.y != o[r][1]) | (e.z != o[r][2]) | (e.w != o[r][3]);
                 if (d.mode & kJobStore)
-                  st_stream(const_cast<uint8_t *>(a.ptrs[d.ptr_off + n_in + d.n_out + r]) + col[v],
+                  st_stream(const_cast<uint8_t *>(ptrs[d.ptr_off + n_in + d.n_out + r]) + col[v],
                             make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]));
               } else {
-                uint8_t *dst = const_cast<uint8_t *>(a.ptrs[d.ptr_off + n_in + r]) + col[v];
+                uint8_t *dst = const_cast<uint8_t *>(ptrs[d.ptr_off + n_in + r]) + col[v];
                 st_stream(dst, make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]));
               }
             }
@@ -295,7 +304,9 @@ struct RegShape {
 };
 
 template <int K, bool VERIFY>
-__global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBlocks) k_apply_reg(ApplyArgs a) {
+__global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBlocks) k_apply_reg(const __grid_constant__ ApplyArgs a) {
+  const JobDesc *const jobs = job_list(a);
+  const uint8_t *const *const ptrs = ptr_list(a);
   using Shape = RegShape<K, VERIFY>;
   constexpr int S = Shape::kStages, W = Shape::kWords;
   constexpr uint32_t kTile = Shape::kTile, kStageBytes = Shape::kSlots * kTile;
@@ -324,12 +335,12 @@ __global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBloc
     uint32_t issued = 0;
     bool ok = true;
     for (uint32_t t = t0; t < t1; ++t) {
-      const JobDesc d = a.jobs[job];
+      const JobDesc d = jobs[job];
       const uint64_t base = uint64_t(tile) * kTile;
       if (base < d.vec_len) {
         const uint32_t valid = uint32_t(d.vec_len - base < kTile ? d.vec_len - base : kTile);
         const uint32_t rows = K + (VERIFY ? d.n_out : 0);
-        const uint8_t *const *ptr = a.ptrs + d.ptr_off;
+        const uint8_t *const *ptr = ptrs + d.ptr_off;
         if (!mbar_wait(ebar + 8 * s, ph ^ 1)) {
           ok = false;
           break;
@@ -364,8 +375,8 @@ __global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBloc
     const uint64_t base = uint64_t(tile) * kTile;
     if (fresh) {
       fresh = false;
-      d = a.jobs[job];
-      const uint8_t *const *out = a.ptrs + d.ptr_off + K + (VERIFY ? d.n_out : 0);
+      d = jobs[job];
+      const uint8_t *const *out = ptrs + d.ptr_off + K + (VERIFY ? d.n_out : 0);
 #pragma unroll
       for (int r = 0; r < 4; ++r)
         dst[r] = uint32_t(r) < d.n_out && (!VERIFY || (d.mode & kJobStore)) ? const_cast<uint8_t *>(out[r]) : nullptr;
@@ -430,15 +441,17 @@ __global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBloc
 // Byte-granular path for the columns past each job's vec_len.  One thread per
 // byte column.
 template <bool VERIFY, bool ACC = false>
-__global__ void k_apply_tail(ApplyArgs a, uint64_t max_tail) {
+__global__ void k_apply_tail(const __grid_constant__ ApplyArgs a, uint64_t max_tail) {
+  const JobDesc *const jobs = job_list(a);
+  const uint8_t *const *const ptrs = ptr_list(a);
   const uint64_t n = max_tail * a.n_jobs;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t job = uint32_t(i / max_tail);
-    const JobDesc d = a.jobs[job];
+    const JobDesc d = jobs[job];
     const uint64_t col = d.vec_len + (i - uint64_t(job) * max_tail);
     if (col >= a.len || (d.mode & kJobUnaligned)) continue;
-    if (apply_column<VERIFY, ACC>(a.ptrs, d, col) && VERIFY) atomicOr(a.flags + d.flag_idx, 1u);
+    if (apply_column<VERIFY, ACC>(ptrs, d, col) && VERIFY) atomicOr(a.flags + d.flag_idx, 1u);
   }
 }
 
@@ -515,16 +528,18 @@ __device__ __forceinline__ void unaligned_mac(uint32_t (*acc)[4], const uint8_t 
 }
 
 template <bool VERIFY, bool ACC>
-__global__ void __launch_bounds__(kApplyThreads + 32, 3) k_apply_unaligned(ApplyArgs a) {
+__global__ void __launch_bounds__(kApplyThreads + 32, 3) k_apply_unaligned(const __grid_constant__ ApplyArgs a) {
+  const JobDesc *const jobs = job_list(a);
+  const uint8_t *const *const ptrs = ptr_list(a);
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint64_t words = a.len >= 12 ? (a.len - 8) / 4 : 0;
   const uint32_t tiles_per_job = uint32_t((words * 4 + kTileU - 1) / kTileU) + (words ? 0 : 1);
   const uint32_t total = tiles_per_job * a.n_jobs;
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const uint32_t job = t / tiles_per_job, tile = t - job * tiles_per_job;
-    const JobDesc d = a.jobs[job];
+    const JobDesc d = jobs[job];
     if (!(d.mode & kJobUnaligned)) continue;  // CTA-uniform
-    const uint8_t *const *ptr = a.ptrs + d.ptr_off;
+    const uint8_t *const *ptr = ptrs + d.ptr_off;
     if (tid >= kApplyThreads) {
       // The last warp, beside the others' words: the at most 11 columns before
       // and after them, two threads each, with the job's first tile.
