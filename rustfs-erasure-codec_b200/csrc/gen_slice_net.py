@@ -133,12 +133,13 @@ def emit_xor(dst, srcs):
     return out
 
 
-def emit_table(bits, q, pairs, nets):
-    name = f"mac{pairs if pairs > 1 else ''}_nibble"
+def emit_table(bits, q, pairs, nets, prefix="mac"):
+    name = f"{prefix}{pairs if pairs > 1 else ''}_nibble"
     nx = bits * pairs
     args = ", ".join(f"uint32_t *x{p}, const uint32_t *y{p}" for p in range(pairs))
     print("template <>")
-    print(f"__device__ __forceinline__ void {name}<{bits}, {4 * q}>(uint32_t n, {args}) {{")
+    targs = f"{bits}, {4 * q}" if prefix == "mac" else f"{4 * q}"
+    print(f"__device__ __forceinline__ void {name}<{targs}>(uint32_t n, {args}) {{")
     print('  asm volatile(')
     most = max(len(t) for _, t in nets[1:])
     print(f'      "{{\\n\\t.reg .b32 t<{most + 1}>;\\n"')
@@ -191,6 +192,18 @@ def main():
             print(f"// GF(2^{bits}), nibble {q}: {total / 15:.1f} XOR instructions a network on average.")
             for pairs in (1, 2):
                 emit_table(bits, q, pairs, nets)
+    # GF(2^16)'s subfield GF(256), which maps each half of the planes to itself.
+    tmul = field(16)
+    for q in range(2):
+        nets = [None]
+        for n in range(1, 16):
+            cols = [tmul(n << (4 * q), 1 << b) for b in range(8)]
+            assert all(c < 256 and tmul(n << (4 * q), 256 << b) == c << 8 for b, c in enumerate(cols))
+            nets.append(network([{b for b in range(8) if (cols[b] >> r) & 1} for r in range(8)], 400, rng))
+        print(f"// GF(256) in GF(2^16), nibble {q}: "
+              f"{sum(cost(*n) for n in nets[1:]) / 15:.1f} XOR instructions a network on average.")
+        for pairs in (1, 2):
+            emit_table(8, q, pairs, nets, "sub")
 
 
 if __name__ == "__main__":

@@ -24,7 +24,8 @@
 // (src/core/leopard_gf16/decode.rs:704-910, encode.rs:109-252).
 //
 // Constants: lane position r + off over distance d as in slice_fft.cuh; below
-// 4096 in A and C (three nibbles), below 256 in B (two).
+// 4096 in A and C (three nibbles), below 256 in B: elements of GF(256), so B works
+// on the two halves of the planes separately (Sub16).
 #pragma once
 
 #include <cuda_runtime.h>

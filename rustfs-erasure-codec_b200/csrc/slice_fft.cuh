@@ -40,21 +40,23 @@ __device__ __forceinline__ void xor_planes(uint32_t *a, const uint32_t *b) {
 }
 // Radix-4 on lanes r, r + d, r + 2d, r + 3d (e, e2: tower constants of the
 // inner and the outer layer).
+template <class F>
 __device__ __forceinline__ void ifft4(uint32_t (*v)[8], uint32_t e, uint32_t e2) {
   xor_planes<8>(v[1], v[0]);
   xor_planes<8>(v[3], v[2]);
-  mac2(e, v[0], v[1], v[2], v[3]);
-  mac_const<8, 2>(v[2], v[3]);
+  F::mac2(e, v[0], v[1], v[2], v[3]);
+  F::beta1(v[2], v[3]);
   xor_planes<8>(v[2], v[0]);
   xor_planes<8>(v[3], v[1]);
-  mac2(e2, v[0], v[2], v[1], v[3]);
+  F::mac2(e2, v[0], v[2], v[1], v[3]);
 }
+template <class F>
 __device__ __forceinline__ void fft4(uint32_t (*v)[8], uint32_t e, uint32_t e2) {
-  mac2(e2, v[0], v[2], v[1], v[3]);
+  F::mac2(e2, v[0], v[2], v[1], v[3]);
   xor_planes<8>(v[2], v[0]);
   xor_planes<8>(v[3], v[1]);
-  mac2(e, v[0], v[1], v[2], v[3]);
-  mac_const<8, 2>(v[2], v[3]);
+  F::mac2(e, v[0], v[1], v[2], v[3]);
+  F::beta1(v[2], v[3]);
   xor_planes<8>(v[1], v[0]);
   xor_planes<8>(v[3], v[2]);
 }
@@ -102,7 +104,7 @@ struct Rows {
 // (src itself, or with acc an accumulator they are XORed into).  Groups at or
 // past `limit` are skipped, and so are groups none of whose 4-lane blocks is
 // in `need` (bit i: lanes 4i..4i+3; ~0 for all).
-template <int WT, bool FWD>
+template <int WT, bool FWD, class F = Gf8>
 __device__ __forceinline__ void slice_pass4(const Rows<WT> &src, const Rows<WT> &dst, bool acc, uint32_t lanes, uint32_t lgd,
                                             uint32_t off, uint32_t limit, uint64_t need) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, d = 1u << lgd;
@@ -111,14 +113,14 @@ __device__ __forceinline__ void slice_pass4(const Rows<WT> &src, const Rows<WT> 
   for (uint32_t q = warp; q < (lanes >> 2); q += warps) {
     const uint32_t r = (q >> lgd) << (lgd + 2), l = r + (q & (d - 1));
     if (r >= limit || !((need >> (r >> 2)) & block)) continue;  // warp-uniform
-    const uint32_t e = tower_const<8>((r + off) >> lgd), e2 = tower_const<8>((r + off) >> (lgd + 1));
+    const uint32_t e = F::tower((r + off) >> lgd), e2 = F::tower((r + off) >> (lgd + 1));
     uint32_t v[4][8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) src.load(src.at(l) + j * (d * Rows<WT>::kStride), v[j]);
     if (FWD)
-      fft4(v, e, e2);
+      fft4<F>(v, e, e2);
     else
-      ifft4(v, e, e2);
+      ifft4<F>(v, e, e2);
     if (!FWD && acc) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) dst.store_xor(dst.at(l) + j * (d * Rows<WT>::kStride), v[j]);
@@ -129,19 +131,19 @@ __device__ __forceinline__ void slice_pass4(const Rows<WT> &src, const Rows<WT> 
   }
 }
 // The leftover layer of an odd log2 size (the topmost one in both directions).
-template <int WT, bool FWD>
+template <int WT, bool FWD, class F = Gf8>
 __device__ __forceinline__ void slice_pass2(const Rows<WT> &src, const Rows<WT> &dst, bool acc, uint32_t lanes, uint32_t lgd,
                                             uint32_t off) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, d = 1u << lgd;
 #pragma unroll 1
   for (uint32_t q = warp; q < (lanes >> 1); q += warps) {
     const uint32_t r = (q >> lgd) << (lgd + 1), l = r + (q & (d - 1));
-    const uint32_t e = tower_const<8>((r + off) >> lgd);
+    const uint32_t e = F::tower((r + off) >> lgd);
     uint32_t x[8], y[8];
     src.load(src.at(l), x);
     src.load(src.at(l + d), y);
     if (!FWD) xor_planes<8>(y, x);
-    mac<8>(e, x, y);
+    F::mac(e, x, y);
     if (FWD) xor_planes<8>(y, x);
     if (!FWD && acc) {
       dst.store_xor(dst.at(l), x);
@@ -155,33 +157,33 @@ __device__ __forceinline__ void slice_pass2(const Rows<WT> &src, const Rows<WT> 
 
 // IFFT over 2^b lanes: radix-4 passes from distance 1 up.  The last pass XORs
 // into dst when acc; with b == 0 there is no pass (the caller placed the row).
-template <int WT>
+template <int WT, class F = Gf8>
 __device__ __forceinline__ void slice_ifft(const Rows<WT> &src, const Rows<WT> &dst, bool acc, uint32_t b, uint32_t off,
                                            uint32_t limit) {
   uint32_t lgd = 0;
 #pragma unroll 1
   for (; lgd + 2 <= b; lgd += 2) {
     const bool last = lgd + 2 == b;
-    slice_pass4<WT, false>(src, last ? dst : src, last && acc, 1u << b, lgd, off, last ? ~0u : limit, ~0ull);
+    slice_pass4<WT, false, F>(src, last ? dst : src, last && acc, 1u << b, lgd, off, last ? ~0u : limit, ~0ull);
     __syncthreads();
   }
   if (lgd < b) {
-    slice_pass2<WT, false>(src, dst, acc, 1u << b, lgd, off);
+    slice_pass2<WT, false, F>(src, dst, acc, 1u << b, lgd, off);
     __syncthreads();
   }
 }
 // FFT over 2^b lanes in place, from the top layer down.
-template <int WT>
+template <int WT, class F = Gf8>
 __device__ __forceinline__ void slice_fft(const Rows<WT> &s, uint32_t b, uint32_t limit, uint64_t need) {
   uint32_t lgd = b;
   if (b & 1) {
-    slice_pass2<WT, true>(s, s, false, 1u << b, --lgd, 0);
+    slice_pass2<WT, true, F>(s, s, false, 1u << b, --lgd, 0);
     __syncthreads();
   }
 #pragma unroll 1
   while (lgd >= 2) {
     lgd -= 2;
-    slice_pass4<WT, true>(s, s, false, 1u << b, lgd, 0, limit, need);
+    slice_pass4<WT, true, F>(s, s, false, 1u << b, lgd, 0, limit, need);
     __syncthreads();
   }
 }
@@ -365,7 +367,7 @@ __device__ __forceinline__ void slice_lane_info(const SliceArgs &a, const LeoJob
 // transform's first, so all its constants are fixed.  A row depends on rows of
 // the same or a larger a, so with a taken in ascending rounds each round reads
 // everything, waits for the CTA, then writes.
-template <int WT>
+template <int WT, class F = Gf8>
 __device__ __forceinline__ void slice_middle(const Rows<WT> &s, uint32_t n) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, items = n >> 2;
   const uint32_t quarter = items * Rows<WT>::kStride;
@@ -378,7 +380,7 @@ __device__ __forceinline__ void slice_middle(const Rows<WT> &s, uint32_t n) {
     for (int j = 0; j < 4; ++j) Rows<WT>::load(base + j * quarter, v[j]);
     xor_planes<8>(v[1], v[0]);  // IFFT_top
     xor_planes<8>(v[3], v[2]);
-    mac_const<8, 2>(v[2], v[3]);
+    F::beta1(v[2], v[3]);
     xor_planes<8>(v[2], v[0]);
     xor_planes<8>(v[3], v[1]);
     xor_planes<8>(v[0], v[1]);  // 1 + N_top
@@ -387,7 +389,7 @@ __device__ __forceinline__ void slice_middle(const Rows<WT> &s, uint32_t n) {
     xor_planes<8>(v[2], v[3]);
     xor_planes<8>(v[2], v[0]);  // FFT_top
     xor_planes<8>(v[3], v[1]);
-    mac_const<8, 2>(v[2], v[3]);
+    F::beta1(v[2], v[3]);
     xor_planes<8>(v[1], v[0]);
     xor_planes<8>(v[3], v[2]);
 #pragma unroll 1
@@ -456,7 +458,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
             v[3][i] = x[i];
           }
         }
-        ifft4(v, tower_const<8>(r), tower_const<8>(r >> 1));
+        ifft4<Gf8>(v, tower_const<8>(r), tower_const<8>(r >> 1));
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) s.store(s.at(r + j), v[j]);
@@ -493,7 +495,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
       uint32_t v[4][8];
 #pragma unroll
       for (int j = 0; j < 4; ++j) Rows<WT>::load(s.at(r + j), v[j]);
-      fft4(v, tower_const<8>(r), tower_const<8>(r >> 1));
+      fft4<Gf8>(v, tower_const<8>(r), tower_const<8>(r >> 1));
 #pragma unroll 1
       for (uint32_t j = 0; j < 4; ++j) {
         const uint64_t ptr = info.ptr[r + j];

@@ -216,6 +216,13 @@ __device__ __forceinline__ void mac_nibble(uint32_t n, uint32_t *x0, const uint3
 template <int BITS, int SH>
 __device__ __forceinline__ void mac2_nibble(uint32_t n, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
                                             const uint32_t *y1);
+// The same for half the planes of GF(2^16) and a constant of its subfield
+// GF(256).
+template <int SH>
+__device__ __forceinline__ void sub_nibble(uint32_t n, uint32_t *x0, const uint32_t *y0);
+template <int SH>
+__device__ __forceinline__ void sub2_nibble(uint32_t n, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
+                                            const uint32_t *y1);
 #include "slice_net.cuh"
 
 // x ^= c * y (one pair, two pairs) for a warp-uniform constant in tower
@@ -229,11 +236,6 @@ __device__ __forceinline__ void mac(uint32_t c, uint32_t *x, const uint32_t *y) 
     mac_nibble<BITS, BITS == 16 ? 12 : 0>((c >> 12) & 15, x, y);
   }
 }
-__device__ __forceinline__ void mac2(uint32_t c, uint32_t *x0, const uint32_t *y0, uint32_t *x1, const uint32_t *y1) {
-  mac2_nibble<8, 0>(c & 15, x0, y0, x1, y1);
-  mac2_nibble<8, 4>(c >> 4, x0, y0, x1, y1);
-}
-
 // Tower coordinates of a Cantor constant, nibble by nibble.
 template <int BITS>
 struct NibbleTower {
@@ -254,6 +256,41 @@ __device__ __forceinline__ uint32_t tower_const(uint32_t e) {
   return c_tower16.v[0][e & 15] ^ c_tower16.v[1][(e >> 4) & 15] ^ c_tower16.v[2][(e >> 8) & 15] ^
          c_tower16.v[3][e >> 12];
 }
+
+// The fields of the 8-plane transforms (slice_fft.cuh): Leopard GF(2^8), and
+// half the planes of GF(2^16) under its subfield GF(256).
+struct Gf8 {
+  __device__ __forceinline__ static uint32_t tower(uint32_t e) { return tower_const<8>(e); }
+  __device__ __forceinline__ static void mac(uint32_t c, uint32_t *x, const uint32_t *y) { rsgpu::mac<8>(c, x, y); }
+  __device__ __forceinline__ static void mac2(uint32_t c, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
+                                              const uint32_t *y1) {
+    mac2_nibble<8, 0>(c & 15, x0, y0, x1, y1);
+    mac2_nibble<8, 4>(c >> 4, x0, y0, x1, y1);
+  }
+  __device__ __forceinline__ static void beta1(uint32_t *x, const uint32_t *y) { mac_const<8, 2>(x, y); }
+};
+struct Sub16 {
+  __device__ __forceinline__ static uint32_t tower(uint32_t e) {
+    return c_tower16.v[0][e & 15] ^ c_tower16.v[1][e >> 4];
+  }
+  __device__ __forceinline__ static void mac(uint32_t c, uint32_t *x, const uint32_t *y) {
+    sub_nibble<0>(c & 15, x, y);
+    sub_nibble<4>(c >> 4, x, y);
+  }
+  __device__ __forceinline__ static void mac2(uint32_t c, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
+                                              const uint32_t *y1) {
+    sub2_nibble<0>(c & 15, x0, y0, x1, y1);
+    sub2_nibble<4>(c >> 4, x0, y0, x1, y1);
+  }
+  __device__ __forceinline__ static void beta1(uint32_t *x, const uint32_t *y) {
+    constexpr PlaneMap<16> net = mul_map<16, 2>();  // closed on the first 8 planes
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+        if ((net.col[b] >> r) & 1) x[r] ^= y[b];
+  }
+};
 
 // Bytes of 8 words -> 8 bit planes, and back: the three swaps exchange one
 // bit of the word index with one bit of the bit index each, so the map is its
