@@ -105,87 +105,114 @@ __global__ void __launch_bounds__(NT, MINB) k_slice16_a(Slice16Args a) {
       }
     }
     __syncthreads();
-    ifft16<3>(sbase, sbase, false, a.bl, DEC ? R : a.m + R, limit - R);
-    uint4 *out = a.v + (size_t(w.x) * a.v_rows + R) * 128 + t;
-#pragma unroll 1
-    for (uint32_t i = warp; i < rows; i += warps) copy_row_out(out + size_t(i) * 128, sbase + i * kRow16);
-    __syncthreads();
+    ifft16<3>(sbase, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, a.bl, DEC ? R : a.m + R, limit - R);
   }
 }
+
+// Half rows in the scratch buffer, `step` uint4 apart: what the first pass of B
+// reads and the last one writes.
+struct ScratchIn {
+  const uint4 *p;
+  size_t step;
+  uint32_t live;  // rows past it are zero
+  __device__ __forceinline__ void get(uint32_t r, uint32_t j, uint32_t *v) const {
+    uint4 x = make_uint4(0, 0, 0, 0), y = x;
+    if (r + j < live) x = p[(r + j) * step], y = p[(r + j) * step + 32];  // warp-uniform
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+  }
+};
+struct FirstRows : Rows<32> {  // a skipped group's rows are zero
+  __device__ __forceinline__ FirstRows(const Rows<32> &r) : Rows<32>(r) {}
+  __device__ __forceinline__ void skip(uint32_t l, uint32_t d) const {
+    const uint32_t zero[8] = {};
+    for (uint32_t j = 0; j < 4; ++j) put(l, j * d, zero);
+  }
+};
+struct ScratchOut {
+  uint4 *p;
+  size_t step;
+  uint32_t rows;  // rows past it are not wanted
+  __device__ __forceinline__ void put(uint32_t r, uint32_t j, const uint32_t *v) const {
+    if (r + j >= rows) return;  // warp-uniform
+    p[(r + j) * step] = make_uint4(v[0], v[1], v[2], v[3]);
+    p[(r + j) * step + 32] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+  __device__ __forceinline__ void skip(uint32_t, uint32_t) const {}
+};
 
 // B: the high layers of residue c (lanes c + 2^bl * j), V -> U.  All constants
 // lie in GF(256), which maps the low and the high 8 planes to themselves, so
 // the two halves of a row are independent 8-plane transforms: half the shared
 // memory and registers of 16-plane rows, twice the warps (1024+512, 16 KiB x 16:
-// encode 535 -> 476 us, rebuild 1279 -> 1110).
+// encode 535 -> 476 us, rebuild 1279 -> 1110).  The first pass reads the scratch
+// buffer and the last one writes it (64 rows: 83 -> 71 us for 64 tiles).
 template <bool DEC>
 __global__ void __launch_bounds__(512, 2) k_slice16_b(Slice16Args a) {
   extern __shared__ __align__(16) uint4 smem16[];
-  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
+  const uint32_t t = threadIdx.x & 31;
   const uint32_t rows = 1u << a.bh, residues = 1u << a.bl, b = a.bh, odd = b & 1;
   const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem16));
-  using Half = Rows<32>;
-  const Half acc(sbase, t), tmp(sbase + rows * Half::kStride, t);
+  const Rows<32> acc(sbase, t), tmp(sbase + rows * Rows<32>::kStride, t);
   const size_t step = size_t(residues) * 128;  // one j on
-  auto fetch = [&](const Half &dst, const uint4 *in, uint32_t live) {
-#pragma unroll 2
-    for (uint32_t j = warp; j < rows; j += warps) {
-      uint4 x = make_uint4(0, 0, 0, 0), y = x;
-      if (j < live) x = in[j * step], y = in[j * step + 32];
-      sts_words(dst.at(j), x);
-      sts_words(dst.at(j) + Half::kHalf, y);
-    }
-    __syncthreads();
-  };
 #pragma unroll 1
   for (uint32_t it = blockIdx.x; it < a.tiles * residues * 2; it += gridDim.x) {
     const Item16 w = item16(a, it >> 1, residues);
     const uint32_t half = (it & 1) * 64 + t;
     const uint4 *vin = a.v + (size_t(w.x) * a.v_rows + w.grp) * 128 + half;
-    uint4 *uout = a.u + (size_t(w.x) * a.u_rows + w.grp) * 128 + half;
-    const uint32_t out = a.u_rows >> a.bl;
+    const ScratchOut uout{a.u + (size_t(w.x) * a.u_rows + w.grp) * 128 + half, step, a.u_rows >> a.bl};
+    uint32_t lgd = 2;  // layers done by the IFFT, then left to the FFT
     if (DEC) {
       const uint32_t live = (a.jobs[w.job].input_count + residues - 1) >> a.bl;  // groups A wrote
-      fetch(acc, vin, live);
       // Layers 0 .. b - 3 (an odd b: layer 2 alone), the middle, and back.
-      uint32_t lgd = 0;
+      slice_pass4<32, false, Sub16>(ScratchIn{vin, step, live}, FirstRows(acc), false, rows, 0, 0, live, ~0ull);
+      __syncthreads();
+      if (odd) {
+        slice_pass2<32, false, Sub16>(acc, acc, false, rows, lgd++, 0);
+        __syncthreads();
+      }
 #pragma unroll 1
-      while (lgd < b - 2) {
-        if (odd && lgd == 2) {
-          slice_pass2<32, false, Sub16>(acc, acc, false, rows, lgd++, 0);
-        } else {
-          slice_pass4<32, false, Sub16>(acc, acc, false, rows, lgd, 0, live, ~0ull);
-          lgd += 2;
-        }
+      for (; lgd < b - 2; lgd += 2) {
+        slice_pass4<32, false, Sub16>(acc, acc, false, rows, lgd, 0, live, ~0ull);
         __syncthreads();
       }
       slice_middle<32, Sub16>(acc, rows);
-#pragma unroll 1
-      while (lgd) {
-        if (odd && lgd == 3) {
-          slice_pass2<32, true, Sub16>(acc, acc, false, rows, --lgd, 0);
-        } else {
-          lgd -= 2;
-          slice_pass4<32, true, Sub16>(acc, acc, false, rows, lgd, 0, out, ~0ull);
-        }
-        __syncthreads();
-      }
     } else {
       const uint32_t groups = (a.k + a.m - 1) / a.m;
 #pragma unroll 1
       for (uint32_t g = 0; g < groups; ++g) {
-        const uint32_t live = min(rows, ((a.k - g * a.m) + residues - 1) >> a.bl);
-        const Half &dst = g ? tmp : acc;
-        fetch(dst, vin + size_t(g) * rows * step, live);
-        slice_ifft<32, Sub16>(dst, acc, g != 0, b, rows * (1 + g), live);
+        const uint32_t live = min(rows, ((a.k - g * a.m) + residues - 1) >> a.bl), off = rows * (1 + g);
+        const Rows<32> &dst = g ? tmp : acc;
+        slice_pass4<32, false, Sub16>(ScratchIn{vin + size_t(g) * rows * step, step, live}, FirstRows(dst), false, rows,
+                                      0, off, live, ~0ull);
+        __syncthreads();
+#pragma unroll 1
+        for (lgd = 2; lgd + 2 <= b; lgd += 2) {
+          const bool last = lgd + 2 == b;
+          slice_pass4<32, false, Sub16>(dst, last ? acc : dst, last && g, rows, lgd, off, last ? ~0u : live, ~0ull);
+          __syncthreads();
+        }
+        if (odd) {
+          slice_pass2<32, false, Sub16>(dst, acc, g != 0, rows, lgd, off);
+          __syncthreads();
+        }
       }
-      slice_fft<32, Sub16>(acc, b, out, ~0ull);
+      if (odd) {
+        slice_pass2<32, true, Sub16>(acc, acc, false, rows, b - 1, 0);
+        __syncthreads();
+      }
+      lgd = b - odd;
     }
-#pragma unroll 2
-    for (uint32_t j = warp; j < out; j += warps) {
-      uout[j * step] = lds_words(acc.at(j));
-      uout[j * step + 32] = lds_words(acc.at(j) + Half::kHalf);
+#pragma unroll 1
+    for (; lgd > 2 + (DEC ? odd : 0u); lgd -= 2) {
+      slice_pass4<32, true, Sub16>(acc, acc, false, rows, lgd - 2, 0, uout.rows, ~0ull);
+      __syncthreads();
     }
+    if (DEC && odd) {
+      slice_pass2<32, true, Sub16>(acc, acc, false, rows, 2, 0);
+      __syncthreads();
+    }
+    slice_pass4<32, true, Sub16>(acc, uout, false, rows, 0, 0, uout.rows, ~0ull);
     __syncthreads();
   }
 }
@@ -226,20 +253,15 @@ __global__ void __launch_bounds__(NT, MINB) k_slice16_c(Slice16Args a) {
       }
     }
     const uint4 *uin = a.u + (size_t(w.x) * a.u_rows + R) * 128 + t;
-    if (MODE == 2) {
-      const bool live = R < jd.input_count;
+    if (MODE == 2 && R < jd.input_count) {  // CTA-uniform
       const uint4 *vin = a.v + (size_t(w.x) * a.v_rows + R) * 128 + t;
-      const uint4 *in = live ? vin : uin;
 #pragma unroll 2
-      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, in + size_t(i) * 128);
+      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, vin + size_t(i) * 128);
       __syncthreads();
-      if (live) derivative16<true>(sbase, rows, uin);
-    } else {
-#pragma unroll 2
-      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, uin + size_t(i) * 128);
-      __syncthreads();
+      derivative16(sbase, rows, uin);
+      uin = nullptr;
     }
-    fft16<3>(sbase, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
+    fft16<3>(sbase, uin, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
     const Cols16 cols(w.col, t, a.len);
     uint32_t bad = 0;
 #pragma unroll 1
@@ -278,13 +300,15 @@ struct Launch16 {
   size_t smem;
   uint32_t groups;  // work items a tile
 };
-// Up to 32 rows (64 KiB): CTAs of 256 threads, one radix-4 group a warp, three
-// an SM at 80 registers.  64 rows: one CTA of 512.
-#define RS_PICK16(K, X) (smem <= 64 * 1024 ? K<X, 256, 2> : K<X, 512, 1>)
+// One radix-4 group a warp at 128 registers, 16 warps an SM: CTAs of 128 threads
+// for 16 rows (256 threads, half of them idle in the passes: 1024+512 encode of
+// 16 KiB x 16 476 us; with this and direct scratch access 370), 256 for 32, 512
+// for 64.
+#define RS_PICK16(K, X) (smem <= 32 * 1024 ? K<X, 128, 4> : smem <= 64 * 1024 ? K<X, 256, 2> : K<X, 512, 1>)
 void launches16(int op, const Slice16Args &a, Launch16 *out) {
   const bool dec = op == RSGPU_OP_RECONSTRUCT;
   auto fill = [&](int i, size_t smem, uint32_t groups, Kernel16 fn) {
-    out[i] = Launch16{fn, smem <= 64 * 1024 ? 256 : 512, smem, groups};
+    out[i] = Launch16{fn, smem <= 32 * 1024 ? 128 : smem <= 64 * 1024 ? 256 : 512, smem, groups};
   };
   size_t smem = size_t(kRow16) << a.bl;
   fill(0, smem, a.v_rows >> a.bl, dec ? RS_PICK16(k_slice16_a, true) : RS_PICK16(k_slice16_a, false));
@@ -306,9 +330,10 @@ uint32_t log2u(uint32_t v) {
 bool slice16_configure(int op, Slice16Args &a) {
   const bool dec = op == RSGPU_OP_RECONSTRUCT;
   const uint32_t b = log2u(dec ? a.n : a.m);
-  // Where this pays (one B200, register-stage / here, us):
-  //   rebuild 1024+512 16 KiB x 16 2424 / 1310, 300+100 671 / 370, 64+32 118 / 93,
-  //   48+16 (64 lanes) 65 / 65;  encode 2048+1024 1868 / 1134, 1024+512 732 / 550,
+  // Where this pays (one B200, register-stage / here, us; all but the first of
+  // each kind with 16-plane high layers):
+  //   rebuild 1024+512 16 KiB x 16 2403 / 1054, 300+100 671 / 370, 64+32 118 / 93,
+  //   48+16 (64 lanes) 65 / 65;  encode 1024+512 730 / 370, 2048+1024 1868 / 1134,
   //   60+200 228 / 94, 512+128 231 / 252, 64+32 38 / 51
   // One-level transforms in shared memory have no scratch traffic, and an
   // encode of few lanes is little else.  Below 1 KiB a row is mostly empty.

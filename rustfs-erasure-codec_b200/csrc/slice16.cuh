@@ -68,22 +68,21 @@ __device__ __forceinline__ void row16_store(uint32_t addr, const uint32_t *v) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) sts_words(addr + q * 512, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
 }
-__device__ __forceinline__ void row16_store_xor(uint32_t addr, const uint32_t *v) {
+// The same in the scratch buffer (p: this thread's words).
+__device__ __forceinline__ void row16_get(const uint4 *p, uint32_t *v) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const uint4 a = lds_words(addr + q * 512);
-    sts_words(addr + q * 512,
-              make_uint4(a.x ^ v[4 * q], a.y ^ v[4 * q + 1], a.z ^ v[4 * q + 2], a.w ^ v[4 * q + 3]));
+    const uint4 a = p[q * 32];
+    v[4 * q] = a.x, v[4 * q + 1] = a.y, v[4 * q + 2] = a.z, v[4 * q + 3] = a.w;
   }
 }
-// Rows in the scratch buffer (p: this thread's words).
+__device__ __forceinline__ void row16_put(uint4 *p, const uint32_t *v) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) p[q * 32] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
 __device__ __forceinline__ void copy_row_in(uint32_t addr, const uint4 *p) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) sts_words(addr + q * 512, p[q * 32]);
-}
-__device__ __forceinline__ void copy_row_out(uint4 *p, uint32_t addr) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) p[q * 32] = lds_words(addr + q * 512);
 }
 __device__ __forceinline__ void zero_row(uint32_t addr) {
 #pragma unroll
@@ -93,12 +92,13 @@ __device__ __forceinline__ void zero_row(uint32_t addr) {
 // One pass over `rows` rows: two layers (radix 4, distances d = 2^lgd and 2d)
 // on rows l, l + d, l + 2d, l + 3d, or with !pair the outer layer alone
 // (distance 2^lgd >= 2) on rows l, l + 1 and their partners.  Positions: row i
-// stands at off + i; a group starting at or past `limit` rows is skipped, and
+// stands at off + i; `in` and `out` (this thread's scratch rows), where not
+// null, replace shared memory; a group starting at or past `limit` rows is skipped, and
 // so is one with no 4-row block in `need`.  Both layers go through one copy of
 // the networks (the loop below), with the middle rows exchanged in between:
 // two copies, 34 KB each, overflowed the instruction cache.
 template <int NQ, bool FWD>
-__device__ __forceinline__ void pass16(uint32_t src, uint32_t dst, bool acc, uint32_t rows, uint32_t lgd, bool pair,
+__device__ __forceinline__ void pass16(uint32_t s, const uint4 *in, uint4 *out, uint32_t rows, uint32_t lgd, bool pair,
                                        uint32_t off, uint32_t limit, uint32_t need) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t d = 1u << lgd, span = pair ? 4 * d : 2 * d;  // rows of a block
@@ -121,7 +121,12 @@ __device__ __forceinline__ void pass16(uint32_t src, uint32_t dst, bool acc, uin
     const uint32_t e_in = tower_const<16>((r + off) >> lgd), e_out = pair ? tower_const<16>((r + off) >> (lgd + 1)) : e_in;
     uint32_t v[4][16];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) row16_load(src + row[j] * kRow16, v[j]);
+    for (int j = 0; j < 4; ++j) {
+      if (in)  // CTA-uniform
+        row16_get(in + row[j] * 128, v[j]);
+      else
+        row16_load(s + row[j] * kRow16, v[j]);
+    }
 #pragma unroll 1
     for (int step = pair ? 0 : 1; step < 2; ++step) {
       const bool inner = FWD ? pair && step == 1 : step == 0;
@@ -149,41 +154,42 @@ __device__ __forceinline__ void pass16(uint32_t src, uint32_t dst, bool acc, uin
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (!FWD && acc)
-        row16_store_xor(dst + row[j] * kRow16, v[j]);
+      if (out)  // CTA-uniform
+        row16_put(out + row[j] * 128, v[j]);
       else
-        row16_store(dst + row[j] * kRow16, v[j]);
+        row16_store(s + row[j] * kRow16, v[j]);
     }
   }
 }
-// IFFT over 2^b rows (b >= 2) in src; the last pass writes (acc: XORs into)
-// dst.
+// IFFT over 2^b rows (b >= 2) in shared memory; the last pass writes out.
 template <int NQ>
-__device__ __forceinline__ void ifft16(uint32_t src, uint32_t dst, bool acc, uint32_t b, uint32_t off, uint32_t limit) {
+__device__ __forceinline__ void ifft16(uint32_t rows, uint4 *out, uint32_t b, uint32_t off, uint32_t limit) {
 #pragma unroll 1
   for (uint32_t lgd = 0; lgd < b; lgd += 2) {
     const bool last = lgd + 2 >= b;
-    pass16<NQ, false>(src, last ? dst : src, last && acc, 1u << b, lgd, lgd + 1 < b, off, last ? ~0u : limit, ~0u);
+    pass16<NQ, false>(rows, nullptr, last ? out : nullptr, 1u << b, lgd, lgd + 1 < b, off, last ? ~0u : limit, ~0u);
     __syncthreads();
   }
 }
+// FFT over 2^b rows into shared memory; the first pass reads `in`, unless null.
 template <int NQ>
-__device__ __forceinline__ void fft16(uint32_t rows, uint32_t b, uint32_t off, uint32_t limit, uint32_t need) {
+__device__ __forceinline__ void fft16(uint32_t rows, const uint4 *in, uint32_t b, uint32_t off, uint32_t limit,
+                                      uint32_t need) {
   const uint32_t odd = b & 1;
 #pragma unroll 1
   for (int lgd = int(b) - 2 + int(odd); lgd >= 0; lgd -= 2) {
     const bool single = odd && lgd == int(b) - 1;
-    pass16<NQ, true>(rows, rows, false, 1u << b, uint32_t(lgd), !single, off, single ? ~0u : limit, single ? ~0u : need);
+    pass16<NQ, true>(rows, in, nullptr, 1u << b, uint32_t(lgd), !single, off, single ? ~0u : limit, single ? ~0u : need);
+    in = nullptr;
     __syncthreads();
   }
 }
 
-// Derivative over n >= 4 rows in place.  A warp takes 4 consecutive rows;
-// a row depends only on rows above it, so with the groups taken in ascending
-// rounds each round reads everything, waits for the CTA, then writes.  SUM: a
-// row's new value is the sum of its sources N W plus its row of `add` (this
-// thread's scratch rows) instead of W + N W.
-template <bool SUM>
+// The derivative's low part over n >= 4 rows in place: a row's new value is the
+// sum of its sources N V plus its row of `add` (this thread's scratch rows).  A
+// warp takes 4 consecutive rows; a row depends only on rows above it, so with
+// the groups taken in ascending rounds each round reads everything, waits for
+// the CTA, then writes.
 __device__ __forceinline__ void derivative16(uint32_t rows, uint32_t n, const uint4 *add) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t items = n >> 2;
@@ -192,29 +198,15 @@ __device__ __forceinline__ void derivative16(uint32_t rows, uint32_t n, const ui
     const uint32_t R = min(i0 + warp, items - 1) << 2;  // past the last: redone, not stored
     const uint32_t base = rows + R * kRow16;
     uint32_t v[4][16], u[16];
-    if (SUM) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 w = add[(R + j) * 128 + q * 32];
-          v[j][4 * q] = w.x, v[j][4 * q + 1] = w.y, v[j][4 * q + 2] = w.z, v[j][4 * q + 3] = w.w;
-        }
-      row16_load(base + kRow16, u);
-      xor_planes<16>(v[0], u);
-      row16_load(base + 2 * kRow16, u);
-      xor_planes<16>(v[0], u);
-      row16_load(base + 3 * kRow16, u);
-      xor_planes<16>(v[1], u);
-      xor_planes<16>(v[2], u);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) row16_load(base + j * kRow16, v[j]);
-      xor_planes<16>(v[0], v[1]);
-      xor_planes<16>(v[0], v[2]);
-      xor_planes<16>(v[1], v[3]);
-      xor_planes<16>(v[2], v[3]);
-    }
+    for (int j = 0; j < 4; ++j) row16_get(add + (R + j) * 128, v[j]);
+    row16_load(base + kRow16, u);
+    xor_planes<16>(v[0], u);
+    row16_load(base + 2 * kRow16, u);
+    xor_planes<16>(v[0], u);
+    row16_load(base + 3 * kRow16, u);
+    xor_planes<16>(v[1], u);
+    xor_planes<16>(v[2], u);
 #pragma unroll 1
     for (uint32_t t = 4; t < n; t <<= 1) {
       if (R & t) continue;  // warp-uniform

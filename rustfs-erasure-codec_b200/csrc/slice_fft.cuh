@@ -91,6 +91,10 @@ struct Rows {
     sts_words(addr, make_uint4(v[0], v[1], v[2], v[3]));
     sts_words(addr + kHalf, make_uint4(v[4], v[5], v[6], v[7]));
   }
+  // Row r + j of a pass; a group that a pass skips.
+  __device__ __forceinline__ void get(uint32_t r, uint32_t j, uint32_t *v) const { load(at(r) + j * kStride, v); }
+  __device__ __forceinline__ void put(uint32_t r, uint32_t j, const uint32_t *v) const { store(at(r) + j * kStride, v); }
+  __device__ __forceinline__ void skip(uint32_t, uint32_t) const {}
   __device__ __forceinline__ void store_xor(uint32_t addr, const uint32_t *v) const {
     uint32_t o[8];
     load(addr, o);
@@ -104,29 +108,37 @@ struct Rows {
 // (src itself, or with acc an accumulator they are XORed into).  Groups at or
 // past `limit` are skipped, and so are groups none of whose 4-lane blocks is
 // in `need` (bit i: lanes 4i..4i+3; ~0 for all).
-template <int WT, bool FWD, class F = Gf8>
-__device__ __forceinline__ void slice_pass4(const Rows<WT> &src, const Rows<WT> &dst, bool acc, uint32_t lanes, uint32_t lgd,
+template <int WT, bool FWD, class F = Gf8, class Src = Rows<WT>, class Dst = Rows<WT>>
+__device__ __forceinline__ void slice_pass4(const Src &src, const Dst &dst, bool acc, uint32_t lanes, uint32_t lgd,
                                             uint32_t off, uint32_t limit, uint64_t need) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, d = 1u << lgd;
   const uint64_t block = d >= 64 ? ~0ull : (1ull << d) - 1;  // 4d lanes as bits of `need`
 #pragma unroll 1
   for (uint32_t q = warp; q < (lanes >> 2); q += warps) {
     const uint32_t r = (q >> lgd) << (lgd + 2), l = r + (q & (d - 1));
-    if (r >= limit || !((need >> (r >> 2)) & block)) continue;  // warp-uniform
+    if (r >= limit || !((need >> (r >> 2)) & block)) {  // warp-uniform
+      dst.skip(l, d);
+      continue;
+    }
     const uint32_t e = F::tower((r + off) >> lgd), e2 = F::tower((r + off) >> (lgd + 1));
     uint32_t v[4][8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) src.load(src.at(l) + j * (d * Rows<WT>::kStride), v[j]);
+    for (int j = 0; j < 4; ++j) src.get(l, j * d, v[j]);
     if (FWD)
       fft4<F>(v, e, e2);
     else
       ifft4<F>(v, e, e2);
-    if (!FWD && acc) {
+    bool done = false;
+    if constexpr (!FWD) {
+      if (acc) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dst.store_xor(dst.at(l) + j * (d * Rows<WT>::kStride), v[j]);
-    } else {
+        for (int j = 0; j < 4; ++j) dst.store_xor(dst.at(l) + j * (d * Rows<WT>::kStride), v[j]);
+        done = true;
+      }
+    }
+    if (!done) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dst.store(dst.at(l) + j * (d * Rows<WT>::kStride), v[j]);
+      for (int j = 0; j < 4; ++j) dst.put(l, j * d, v[j]);
     }
   }
 }
