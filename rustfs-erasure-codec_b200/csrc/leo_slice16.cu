@@ -65,6 +65,34 @@ struct Lanes16 {
   }
 };
 
+// An encode's data lanes straight into the first pass, four in flight at once
+// (75 -> 72 us a chunk of 64 tiles of 1024+512).  A decode goes through shared
+// memory, lane by lane: the scaling and the absent third of the lanes cost more
+// in the pass (88 us a chunk; 102 in the pass, more with absent lanes skipped).
+struct DataRows {
+  const Slice16Args &a;
+  const LeoJob &jd;
+  uint32_t R;
+  Cols16 cols;
+  __device__ __forceinline__ void get(const uint32_t *row, uint32_t (*v)[16]) const {
+    const Lanes16 lanes = Lanes16::get<0>(a, jd, R + row[0] + (threadIdx.x & 3));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cols.load(reinterpret_cast<const uint8_t *>(lanes.at(j).ptr), v[j]);
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      Cols16::planes(v[0]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t x = v[0][i];
+        v[0][i] = v[1][i];
+        v[1][i] = v[2][i];
+        v[2][i] = v[3][i];
+        v[3][i] = x;
+      }
+    }
+  }
+};
+
 // A: low IFFT of 2^bl consecutive lanes, shards -> V.  Decode: lane l is
 // parity l or data l - m, scaled by its locator.  Encode: lane l is data l,
 // at position m + l.
@@ -82,30 +110,28 @@ __global__ void __launch_bounds__(NT, MINB) k_slice16_a(Slice16Args a) {
     const uint32_t R = w.grp << a.bl, limit = DEC ? jd.input_count : a.k;
     if (R >= limit) continue;  // CTA-uniform: zero lanes, never read
     const Cols16 cols(w.col, t, a.len);
+    if (DEC) {
 #pragma unroll 1
-    for (uint32_t i0 = 0; i0 < rows; i0 += 32) {
-      const Lanes16 lanes = Lanes16::get<DEC ? 1 : 0>(a, jd, R + i0 + t);
+      for (uint32_t i0 = 0; i0 < rows; i0 += 32) {
+        const Lanes16 lanes = Lanes16::get<1>(a, jd, R + i0 + t);
 #pragma unroll 1
-      for (uint32_t i = warp; i < min(rows - i0, 32u); i += warps) {
-        const Lanes16 lane = lanes.at(i);
-        const uint32_t row = sbase + (i0 + i) * kRow16;
-        if (lane.ptr) {  // warp-uniform
-          uint32_t y[16];
-          cols.load(reinterpret_cast<const uint8_t *>(lane.ptr), y);
-          if (DEC) {
-            uint32_t x[16] = {};
+        for (uint32_t i = warp; i < min(rows - i0, 32u); i += warps) {
+          const Lanes16 lane = lanes.at(i);
+          uint32_t x[16] = {};
+          if (lane.ptr) {  // warp-uniform
+            uint32_t y[16];
+            cols.load(reinterpret_cast<const uint8_t *>(lane.ptr), y);
+            Cols16::planes(y);
             mac16<4>(lane.c, x, y);
-            row16_store(row, x);
-          } else {
-            row16_store(row, y);
           }
-        } else {
-          zero_row(row);
+          row16_store(sbase + (i0 + i) * kRow16, x);
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
-    ifft16<3>(sbase, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, a.bl, DEC ? R : a.m + R, limit - R);
+    const DataRows in{a, jd, R, cols};
+    ifft16<3>(sbase, DEC ? nullptr : &in, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, a.bl, DEC ? R : a.m + R,
+              limit - R);
   }
 }
 
@@ -146,7 +172,7 @@ struct ScratchOut {
 // the two halves of a row are independent 8-plane transforms: half the shared
 // memory and registers of 16-plane rows, twice the warps (1024+512, 16 KiB x 16:
 // encode 535 -> 476 us, rebuild 1279 -> 1110).  The first pass reads the scratch
-// buffer and the last one writes it (64 rows: 83 -> 71 us for 64 tiles).
+// buffer and the last one writes it (64 rows: 83 -> 71 us a chunk of 64 tiles).
 template <bool DEC>
 __global__ void __launch_bounds__(512, 2) k_slice16_b(Slice16Args a) {
   extern __shared__ __align__(16) uint4 smem16[];
@@ -252,16 +278,10 @@ __global__ void __launch_bounds__(NT, MINB) k_slice16_c(Slice16Args a) {
         continue;
       }
     }
-    const uint4 *uin = a.u + (size_t(w.x) * a.u_rows + R) * 128 + t;
-    if (MODE == 2 && R < jd.input_count) {  // CTA-uniform
-      const uint4 *vin = a.v + (size_t(w.x) * a.v_rows + R) * 128 + t;
-#pragma unroll 2
-      for (uint32_t i = warp; i < rows; i += warps) copy_row_in(sbase + i * kRow16, vin + size_t(i) * 128);
-      __syncthreads();
-      derivative16(sbase, rows, uin);
-      uin = nullptr;
-    }
-    fft16<3>(sbase, uin, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
+    const ScratchRows uin{a.u + (size_t(w.x) * a.u_rows + R) * 128 + t};
+    const bool derive = MODE == 2 && R < jd.input_count;  // CTA-uniform; past it V is zero
+    if (derive) derivative16(sbase, rows, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, uin.p);
+    fft16<3>(sbase, derive ? nullptr : &uin, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
     const Cols16 cols(w.col, t, a.len);
     uint32_t bad = 0;
 #pragma unroll 1
@@ -332,8 +352,8 @@ bool slice16_configure(int op, Slice16Args &a) {
   const uint32_t b = log2u(dec ? a.n : a.m);
   // Where this pays (one B200, register-stage / here, us; all but the first of
   // each kind with 16-plane high layers):
-  //   rebuild 1024+512 16 KiB x 16 2403 / 1054, 300+100 671 / 370, 64+32 118 / 93,
-  //   48+16 (64 lanes) 65 / 65;  encode 1024+512 730 / 370, 2048+1024 1868 / 1134,
+  //   rebuild 1024+512 16 KiB x 16 2403 / 1016, 300+100 671 / 370, 64+32 118 / 93,
+  //   48+16 (64 lanes) 65 / 65;  encode 1024+512 730 / 360, 2048+1024 1868 / 1134,
   //   60+200 228 / 94, 512+128 231 / 252, 64+32 38 / 51
   // One-level transforms in shared memory have no scratch traffic, and an
   // encode of few lanes is little else.  Below 1 KiB a row is mostly empty.

@@ -80,9 +80,17 @@ __device__ __forceinline__ void row16_put(uint4 *p, const uint32_t *v) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) p[q * 32] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
+struct ScratchRows {
+  const uint4 *p;
+  __device__ __forceinline__ void get(const uint32_t *row, uint32_t (*v)[16]) const {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) row16_get(p + row[j] * 128, v[j]);
+  }
+};
 __device__ __forceinline__ void copy_row_in(uint32_t addr, const uint4 *p) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) sts_words(addr + q * 512, p[q * 32]);
+  for (int q = 0; q < 4; ++q)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(addr + q * 512), "l"(p + q * 32) : "memory");
 }
 __device__ __forceinline__ void zero_row(uint32_t addr) {
 #pragma unroll
@@ -92,13 +100,13 @@ __device__ __forceinline__ void zero_row(uint32_t addr) {
 // One pass over `rows` rows: two layers (radix 4, distances d = 2^lgd and 2d)
 // on rows l, l + d, l + 2d, l + 3d, or with !pair the outer layer alone
 // (distance 2^lgd >= 2) on rows l, l + 1 and their partners.  Positions: row i
-// stands at off + i; `in` and `out` (this thread's scratch rows), where not
-// null, replace shared memory; a group starting at or past `limit` rows is skipped, and
+// stands at off + i; where not null, `in` gives the rows (an IFFT's skipped ones
+// are zero) and `out` (this thread's scratch rows) takes them; a group starting at or past `limit` rows is skipped, and
 // so is one with no 4-row block in `need`.  Both layers go through one copy of
 // the networks (the loop below), with the middle rows exchanged in between:
 // two copies, 34 KB each, overflowed the instruction cache.
-template <int NQ, bool FWD>
-__device__ __forceinline__ void pass16(uint32_t s, const uint4 *in, uint4 *out, uint32_t rows, uint32_t lgd, bool pair,
+template <int NQ, bool FWD, class In>
+__device__ __forceinline__ void pass16(uint32_t s, const In *in, uint4 *out, uint32_t rows, uint32_t lgd, bool pair,
                                        uint32_t off, uint32_t limit, uint32_t need) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t d = 1u << lgd, span = pair ? 4 * d : 2 * d;  // rows of a block
@@ -117,15 +125,18 @@ __device__ __forceinline__ void pass16(uint32_t s, const uint4 *in, uint4 *out, 
       const uint32_t l = r + 2 * (q & (d / 2 - 1));
       row[0] = l, row[1] = l + d, row[2] = l + 1, row[3] = l + d + 1;
     }
-    if (r >= limit || !((need >> (r >> 2)) & block)) continue;  // warp-uniform
+    if (r >= limit || !((need >> (r >> 2)) & block)) {  // warp-uniform
+      if (!FWD && in)
+        for (int j = 0; j < 4; ++j) zero_row(s + row[j] * kRow16);
+      continue;
+    }
     const uint32_t e_in = tower_const<16>((r + off) >> lgd), e_out = pair ? tower_const<16>((r + off) >> (lgd + 1)) : e_in;
     uint32_t v[4][16];
+    if (in) {  // CTA-uniform
+      in->get(row, v);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (in)  // CTA-uniform
-        row16_get(in + row[j] * 128, v[j]);
-      else
-        row16_load(s + row[j] * kRow16, v[j]);
+      for (int j = 0; j < 4; ++j) row16_load(s + row[j] * kRow16, v[j]);
     }
 #pragma unroll 1
     for (int step = pair ? 0 : 1; step < 2; ++step) {
@@ -161,19 +172,22 @@ __device__ __forceinline__ void pass16(uint32_t s, const uint4 *in, uint4 *out, 
     }
   }
 }
-// IFFT over 2^b rows (b >= 2) in shared memory; the last pass writes out.
-template <int NQ>
-__device__ __forceinline__ void ifft16(uint32_t rows, uint4 *out, uint32_t b, uint32_t off, uint32_t limit) {
+// IFFT over 2^b rows (b >= 3); the first pass reads `in`, unless null, the
+// last one writes out, shared memory is in between.
+template <int NQ, class In>
+__device__ __forceinline__ void ifft16(uint32_t rows, const In *in, uint4 *out, uint32_t b, uint32_t off,
+                                       uint32_t limit) {
 #pragma unroll 1
   for (uint32_t lgd = 0; lgd < b; lgd += 2) {
     const bool last = lgd + 2 >= b;
-    pass16<NQ, false>(rows, nullptr, last ? out : nullptr, 1u << b, lgd, lgd + 1 < b, off, last ? ~0u : limit, ~0u);
+    pass16<NQ, false>(rows, lgd ? nullptr : in, last ? out : nullptr, 1u << b, lgd, lgd + 1 < b, off,
+                      last ? ~0u : limit, ~0u);
     __syncthreads();
   }
 }
 // FFT over 2^b rows into shared memory; the first pass reads `in`, unless null.
 template <int NQ>
-__device__ __forceinline__ void fft16(uint32_t rows, const uint4 *in, uint32_t b, uint32_t off, uint32_t limit,
+__device__ __forceinline__ void fft16(uint32_t rows, const ScratchRows *in, uint32_t b, uint32_t off, uint32_t limit,
                                       uint32_t need) {
   const uint32_t odd = b & 1;
 #pragma unroll 1
@@ -185,44 +199,45 @@ __device__ __forceinline__ void fft16(uint32_t rows, const uint4 *in, uint32_t b
   }
 }
 
-// The derivative's low part over n >= 4 rows in place: a row's new value is the
-// sum of its sources N V plus its row of `add` (this thread's scratch rows).  A
-// warp takes 4 consecutive rows; a row depends only on rows above it, so with
-// the groups taken in ascending rounds each round reads everything, waits for
-// the CTA, then writes.
-__device__ __forceinline__ void derivative16(uint32_t rows, uint32_t n, const uint4 *add) {
-  const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const uint32_t items = n >> 2;
-#pragma unroll 1
-  for (uint32_t i0 = 0; i0 < items; i0 += warps) {
-    const uint32_t R = min(i0 + warp, items - 1) << 2;  // past the last: redone, not stored
-    const uint32_t base = rows + R * kRow16;
-    uint32_t v[4][16], u[16];
+// The derivative's low part over the n >= 4 rows of `in` (this thread's scratch
+// rows): N V + add, into shared memory.  A warp takes 4 consecutive rows; `add`
+// is on its way while the rows it needs of the other warps are copied.  A CTA
+// has a warp for every 4 rows.
+__device__ __forceinline__ void derivative16(uint32_t rows, uint32_t n, const uint4 *in, const uint4 *add) {
+  const uint32_t warp = threadIdx.x >> 5, items = n >> 2;
+  const uint32_t R = min(warp, items - 1) << 2;  // past the last: redone, not stored
+  const uint32_t base = rows + R * kRow16;
+  if (warp < items) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) row16_get(add + (R + j) * 128, v[j]);
-    row16_load(base + kRow16, u);
-    xor_planes<16>(v[0], u);
-    row16_load(base + 2 * kRow16, u);
-    xor_planes<16>(v[0], u);
-    row16_load(base + 3 * kRow16, u);
-    xor_planes<16>(v[1], u);
-    xor_planes<16>(v[2], u);
-#pragma unroll 1
-    for (uint32_t t = 4; t < n; t <<= 1) {
-      if (R & t) continue;  // warp-uniform
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        row16_load(base + (t + j) * kRow16, u);
-        xor_planes<16>(v[j], u);
-      }
-    }
-    __syncthreads();
-    if (i0 + warp < items) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) row16_store(base + j * kRow16, v[j]);
-    }
-    __syncthreads();
+    for (int j = 0; j < 4; ++j) copy_row_in(base + j * kRow16, in + (R + j) * 128);
   }
+  uint32_t v[4][16], u[16];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) row16_get(add + (R + j) * 128, v[j]);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  row16_load(base + kRow16, u);
+  xor_planes<16>(v[0], u);
+  row16_load(base + 2 * kRow16, u);
+  xor_planes<16>(v[0], u);
+  row16_load(base + 3 * kRow16, u);
+  xor_planes<16>(v[1], u);
+  xor_planes<16>(v[2], u);
+#pragma unroll 1
+  for (uint32_t t = 4; t < n; t <<= 1) {
+    if (R & t) continue;  // warp-uniform
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      row16_load(base + (t + j) * kRow16, u);
+      xor_planes<16>(v[j], u);
+    }
+  }
+  __syncthreads();
+  if (warp < items) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) row16_store(base + j * kRow16, v[j]);
+  }
+  __syncthreads();
 }
 
 // A thread's 32 elements of a tile: low and high bytes of half h of blocks
@@ -241,10 +256,12 @@ struct Cols16 {
     uint4 x[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[i] = make_uint4(0, 0, 0, 0);
-    if (on_a) x[0] = ld_stream(p + a), x[2] = ld_stream(p + a + 32);
-    if (on_b) x[1] = ld_stream(p + b), x[3] = ld_stream(p + b + 32);
+    if (p && on_a) x[0] = ld_stream(p + a), x[2] = ld_stream(p + a + 32);
+    if (p && on_b) x[1] = ld_stream(p + b), x[3] = ld_stream(p + b + 32);
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[4 * i] = x[i].x, v[4 * i + 1] = x[i].y, v[4 * i + 2] = x[i].z, v[4 * i + 3] = x[i].w;
+  }
+  __device__ __forceinline__ static void planes(uint32_t *v) {
     slice8(v);
     slice8(v + 8);
     planes_to_tower<16>(v);
