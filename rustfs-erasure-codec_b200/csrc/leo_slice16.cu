@@ -96,8 +96,8 @@ struct DataRows {
 // A: low IFFT of 2^bl consecutive lanes, shards -> V.  Decode: lane l is
 // parity l or data l - m, scaled by its locator.  Encode: lane l is data l,
 // at position m + l.
-template <bool DEC, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_slice16_a(Slice16Args a) {
+template <bool DEC>
+__global__ void __launch_bounds__(512, 1) k_slice16_a(Slice16Args a) {
   extern __shared__ __align__(16) uint4 smem16[];
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
   const uint32_t rows = 1u << a.bl;
@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(512, 2) k_slice16_b(Slice16Args a) {
 
 // C: low FFT of 2^bl consecutive lanes, U (decode: plus N_low V) -> outputs.
 // MODE: 0 encode, 1 verify, 2 decode.
-template <int MODE, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_slice16_c(Slice16Args a) {
+template <int MODE>
+__global__ void __launch_bounds__(512, 1) k_slice16_c(Slice16Args a) {
   extern __shared__ __align__(16) uint4 smem16[];
   __shared__ uint32_t s_need;
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, t = threadIdx.x & 31;
@@ -320,24 +320,19 @@ struct Launch16 {
   size_t smem;
   uint32_t groups;  // work items a tile
 };
-// One radix-4 group a warp at 128 registers, 16 warps an SM: CTAs of 128 threads
-// for 16 rows (256 threads, half of them idle in the passes: 1024+512 encode of
-// 16 KiB x 16 476 us; with this and direct scratch access 370), 256 for 32, 512
-// for 64.
-#define RS_PICK16(K, X) (smem <= 32 * 1024 ? K<X, 128, 4> : smem <= 64 * 1024 ? K<X, 256, 2> : K<X, 512, 1>)
+// One warp for every radix-4 group.  A and C hold 128 registers a thread, so 16
+// warps an SM, in CTAs of 1 (4 rows) to 16 warps (64 rows).  With CTAs of 8 warps
+// for 16 rows, half of them idle in the passes, 1024+512 encode of 16 KiB x 16
+// took 476 us; with 4 warps and direct scratch access 370.
 void launches16(int op, const Slice16Args &a, Launch16 *out) {
   const bool dec = op == RSGPU_OP_RECONSTRUCT;
-  auto fill = [&](int i, size_t smem, uint32_t groups, Kernel16 fn) {
-    out[i] = Launch16{fn, smem <= 32 * 1024 ? 128 : smem <= 64 * 1024 ? 256 : 512, smem, groups};
-  };
-  size_t smem = size_t(kRow16) << a.bl;
-  fill(0, smem, a.v_rows >> a.bl, dec ? RS_PICK16(k_slice16_a, true) : RS_PICK16(k_slice16_a, false));
-  fill(2, smem, a.u_rows >> a.bl, dec ? RS_PICK16(k_slice16_c, 2)
-                                  : op == RSGPU_OP_VERIFY ? RS_PICK16(k_slice16_c, 1) : RS_PICK16(k_slice16_c, 0));
-  smem = (size_t(kRow16 / 2) << a.bh) * (dec || a.k <= a.m ? 1 : 2);
-  out[1] = Launch16{dec ? k_slice16_b<true> : k_slice16_b<false>, int(std::max(32u << a.bh >> 2, 32u)), smem, 2u << a.bl};
+  const int low = 32 << a.bl >> 2, high = 32 << a.bh >> 2;
+  const size_t smem = size_t(kRow16) << a.bl, half = size_t(kRow16 / 2) << a.bh;
+  out[0] = Launch16{dec ? k_slice16_a<true> : k_slice16_a<false>, low, smem, a.v_rows >> a.bl};
+  out[1] = Launch16{dec ? k_slice16_b<true> : k_slice16_b<false>, high, dec || a.k <= a.m ? half : 2 * half, 2u << a.bl};
+  out[2] = Launch16{dec ? k_slice16_c<2> : op == RSGPU_OP_VERIFY ? k_slice16_c<1> : k_slice16_c<0>, low, smem,
+                    a.u_rows >> a.bl};
 }
-#undef RS_PICK16
 
 uint32_t log2u(uint32_t v) {
   uint32_t b = 0;
@@ -350,15 +345,16 @@ uint32_t log2u(uint32_t v) {
 bool slice16_configure(int op, Slice16Args &a) {
   const bool dec = op == RSGPU_OP_RECONSTRUCT;
   const uint32_t b = log2u(dec ? a.n : a.m);
-  // Where this pays (one B200, register-stage / here, us; all but the first of
-  // each kind with 16-plane high layers):
-  //   rebuild 1024+512 16 KiB x 16 2403 / 1016, 300+100 671 / 370, 64+32 118 / 93,
-  //   48+16 (64 lanes) 65 / 65;  encode 1024+512 730 / 360, 2048+1024 1868 / 1134,
-  //   60+200 228 / 94, 512+128 231 / 252, 64+32 38 / 51
-  // One-level transforms in shared memory have no scratch traffic, and an
-  // encode of few lanes is little else.  Below 1 KiB a row is mostly empty.
-  if (b < (dec ? 7 : 8) || a.len < 1024) return false;
-  a.bl = dec ? b / 2 : std::max(b / 2, b > 5 ? b - 5 : 0u);
+  // Where this pays (one B200, register-stage / here, us):
+  //   rebuild 1024+512 16 KiB x 16 2412 / 1018, 300+100 674 / 251, 64+32 118 / 61,
+  //   48+16 (64 lanes) 66 / 40, 40+16 16 KiB x 1 44 / 27, 1 KiB x 32 44 / 30;
+  //   encode 2048+1024 16 KiB x 16 1882 / 858, 1024+512 735 / 360, 60+200 232 / 71,
+  //   512+128 234 / 146, 200+60 (64 lanes) 111 / 67, 16 KiB x 1 33 / 31,
+  //   2 KiB x 16 34 / 30, but 1 KiB x 64 39 / 42 and 512+128 71 / 76.
+  // Below 64 lanes there is too little to split, and a row (2 KiB of a
+  // shard) is half empty at 1 KiB.
+  if (b < 6 || a.len < (dec || b > 7 ? 1024u : 2048u)) return false;
+  a.bl = dec ? std::min(b / 2, b - 4) : std::max(b / 2, b - 5);
   a.bh = b - a.bl;
   if (a.bl > 6 || a.bh > 6) return false;
   const uint32_t low = 1u << a.bl;

@@ -33,6 +33,11 @@ def _setup(k, m, length, stripes, seed):
     (1100, 512, 4096, 1),    # three groups
     (2048, 1024, 1088, 1),   # 4096-lane decode
     (600, 1024, 1024, 1),    # fewer data than parity lanes
+    (200, 60, 2112, 2),      # 64 lanes, four groups
+    (30, 33, 2048, 2),       # 64 lanes, one partial group
+    (200, 100, 4096, 1),     # 128 lanes
+    (250, 100, 1024, 2),     # 128 lanes, shards too short: register-stage kernels
+    (300, 20, 2048, 2),      # 32 lanes: register-stage kernels
 ])
 def test_encode_and_verify(k, m, length, stripes):
     torch, codec, rng, host, buf, ptrs = _setup(k, m, length, stripes, k + m)
@@ -60,7 +65,9 @@ def test_encode_and_verify(k, m, length, stripes):
     (900, 90, 1024, 1),      # 1024 lanes
     (1024, 512, 4160, 1),    # 2048 lanes
     (2048, 1024, 1088, 1),   # 4096 lanes: 64-row levels
-    (40, 16, 2048, 2),       # 64 lanes: register-stage kernels
+    (40, 16, 2048, 2),       # 64 lanes: 4-row low levels
+    (20, 33, 1088, 2),       # the fewest lanes, more parity than data
+    (20, 12, 2048, 2),       # 32 lanes: register-stage kernels
     (3500, 600, 1024, 1),    # 8192 lanes: register-stage kernels
 ])
 def test_reconstruct(k, m, length, stripes):
