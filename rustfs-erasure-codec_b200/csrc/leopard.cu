@@ -1069,12 +1069,14 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
     sa.mod = a.mod;
     sa.max_scratch = L.own_scratch ? kStreamScratch16 : kSlabScratch16;
     if (slice16_configure(op, sa)) {
-      L.sliced16 = true;
-      if (!L.own_scratch) {
-        int rc = grow_scratch(st, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs));
-        if (rc) return rc;
+      if (L.own_scratch) {
+        L.sliced16 = true;
+      } else if (grow_scratch(st, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs)) == RSGPU_OK) {
         std::lock_guard<std::mutex> g(st.scratch_mu);
         L.scratch16 = st.scratch;
+        L.sliced16 = true;
+      } else {
+        cudaGetLastError();  // no room: the register-stage kernels
       }
     }
   }
