@@ -688,7 +688,7 @@ def main():
                        "stripes_per_geometry": args.stripes, "ops_per_step": "encode, reconstruct, verify",
                        "bytes_per_step_per_gpu": total_bytes, "flush": "inputs (137 GiB/GPU) larger than L2",
                        "parallelism": f"stripes x{world} (weak, no collective)"},
-            "roofline": {"bound": "hbm", "kernel": "k_apply_tma (10+4 encode, 4096 x 1 MiB)",
+            "roofline": {"bound": "hbm", "kernel": "k_apply_reg (10+4 encode, 4096 x 1 MiB)",
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "peak_source": peak_kind,
                          "frac_of_nominal_8tbs": round(achieved / 8000.0, 4),

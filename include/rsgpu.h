@@ -331,9 +331,11 @@ int32_t rsgpu_reconstruct_stream_from(const rsgpu_codec *codec, size_t n_shards,
 
 /* ------------------------------------------------------------ mixed batches */
 /* A mixed batch runs many stripes of different codecs (classic GF(2^8),
- * Leopard GF(2^8) / GF(2^16)), shard lengths and operations in ONE persistent
- * kernel over a device work queue of column tiles, optionally launched
- * through a captured CUDA graph.  Like a prepared batch it is planned once and
+ * Leopard GF(2^8) / GF(2^16)), shard lengths and operations in a persistent
+ * kernel over a device work queue of column tiles, plus one launch per codec
+ * and operation for Leopard GF(2^8) work that its own kernels run faster
+ * (planners TABLE and MODEL), optionally launched through a captured CUDA
+ * graph.  Like a prepared batch it is planned once and
  * launched any number of times without allocating or synchronizing; shard
  * pointers are device pointers that must stay valid, and every codec must
  * outlive the batch.  Each operation gets a plan (algorithm, tile); every plan

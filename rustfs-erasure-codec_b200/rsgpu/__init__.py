@@ -522,7 +522,8 @@ def _mix_ops(ops, keep):
 
 class MixedBatch:
     """A mixed batch (rsgpu_mix_prepare in include/rsgpu.h): operations of
-    different codecs, shard lengths and kinds in one persistent kernel.
+    different codecs, shard lengths and kinds in one persistent kernel (large
+    Leopard GF(2^8) work in launches of its own).
 
     ``ops`` is a list of dicts with keys ``codec`` (ReedSolomon), ``op``
     ("encode" / "reconstruct" / "verify"), ``shards`` (k + m device pointers,
