@@ -37,12 +37,11 @@ static_assert(sizeof(JobDesc) == 32, "JobDesc layout");
 // Packed table layout for one coefficient matrix of n_out x n_in: for each
 // group g of 4 outputs and each input j, kTableWords words (byte r of a word
 // belongs to output 4g+r):
-//   [0, 16)   c * n          n = 0..15   (4+4 split: low nibble)
-//   [16, 32)  c * (n << 4)   n = 0..15   (4+4 split: high nibble)
-//   [32, 64)  c * i          i = 0..31   (5+3 split: low five bits)
-//   [64, 72)  for output r: words 64+2r, 65+2r hold the bytes c_r * (h << 5),
-//             h = 0..7        (5+3 split: high three bits, one byte per h)
-constexpr int kTableWords = 72;
+//   [0, 16)   c * n          n = 0..15   (low nibble)
+//   [16, 32)  c * (n << 4)   n = 0..15   (high nibble; every other entry: high
+//                                         three bits)
+//   [32, 64)  c * i          i = 0..31   (low five bits)
+constexpr int kTableWords = 64;
 inline size_t packed_table_words(size_t n_out, size_t n_in) {
   return ((n_out + 3) / 4) * n_in * kTableWords;
 }

@@ -278,7 +278,6 @@ void pack_tables_with(const uint8_t (*mul)[256], const uint8_t *rows, size_t n_o
           t[16 + n] |= uint32_t(mul[c][n << 4]) << (8 * r);
         }
         for (unsigned i = 0; i < 32; ++i) t[32 + i] |= uint32_t(mul[c][i]) << (8 * r);
-        for (unsigned h = 0; h < 8; ++h) t[64 + 2 * r + (h >> 2)] |= uint32_t(mul[c][h << 5]) << (8 * (h & 3));
       }
     }
 }

@@ -727,16 +727,10 @@ __global__ void __launch_bounds__(256) k_decode_tables(DecodeTableArgs a) {
   for (int i = threadIdx.x; i < groups * k * kTableWords; i += blockDim.x) {
     const int e = i % kTableWords, j = (i / kTableWords) % k, g = (i / kTableWords) / k;
     uint32_t word = 0;
-    if (e < 64) {
-      const uint8_t x = e < 16 ? uint8_t(e) : e < 32 ? uint8_t((e - 16) << 4) : uint8_t(e - 32);
-      for (int r = 0; r < 4; ++r) {
-        const int o = g * 4 + r;
-        if (o < n_out) word |= uint32_t(gf.mul(rows[o * k + j], x)) << (8 * r);
-      }
-    } else {
-      const int r = (e - 64) >> 1, h0 = ((e - 64) & 1) * 4, o = g * 4 + r;
-      if (o < n_out)
-        for (int h = 0; h < 4; ++h) word |= uint32_t(gf.mul(rows[o * k + j], uint8_t((h0 + h) << 5))) << (8 * h);
+    const uint8_t x = e < 16 ? uint8_t(e) : e < 32 ? uint8_t((e - 16) << 4) : uint8_t(e - 32);
+    for (int r = 0; r < 4; ++r) {
+      const int o = g * 4 + r;
+      if (o < n_out) word |= uint32_t(gf.mul(rows[o * k + j], x)) << (8 * r);
     }
     out[i] = word;
   }

@@ -1865,12 +1865,8 @@ __global__ void __launch_bounds__(256) k_pack_dense8(const uint8_t *units, uint3
         word |= uint32_t(row[w]) << (8 * r);
       else if (w < 32)
         word |= uint32_t(row[(w - 16) << 4]) << (8 * r);
-      else if (w < 64)
+      else
         word |= uint32_t(row[w - 32]) << (8 * r);
-      else if (((w - 64) >> 1) == r) {
-        const uint32_t h0 = 4 * ((w - 64) & 1);
-        for (uint32_t b = 0; b < 4; ++b) word |= uint32_t(row[(h0 + b) << 5]) << (8 * b);
-      }
     }
     out[x] = word;
   }
