@@ -432,6 +432,22 @@ struct RetiredBlock {
 constexpr size_t kLocatorCacheBytes = size_t(32) << 20;
 constexpr size_t kLocatorCacheMinPlans = 64;
 
+// A device buffer that launches on any stream use in turn: each waits for the
+// previous user's event, then records its own.  An outgrown buffer that a built
+// launch may still use is retired: freed with the codec, never under the launch.
+struct Slab {
+  std::mutex mu;
+  void *ptr = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t done = nullptr;
+  std::vector<void *> retired;
+  ~Slab() {  // the codec's launches have finished
+    for (void *p : retired) cudaFreeAsync(p, cudaStreamPerThread);  // back to the library's pool
+    if (ptr) cudaFreeAsync(ptr, cudaStreamPerThread);
+    if (done) cudaEventDestroy(done);
+  }
+};
+
 struct LeopardState {
   LeoField *field = nullptr;
   uint32_t m = 0, n = 0, mtrunc = 0, last = 0;
@@ -442,18 +458,17 @@ struct LeopardState {
   size_t plan_budget = 0;           // bytes the cached plans may hold
   rsgpu_cache_stats plan_stats{};   // requests, hits, misses, inserts, evictions
   uint64_t build_seq = 0;           // id of the build in progress (under mu)
-  std::vector<void *> owned;    // retired scratch slabs, freed with the codec
   // Locator blocks are carved from these slabs, so a new pattern costs no
   // cudaMalloc once the pool has grown to the cache's budget.
   std::vector<void *> plan_slabs;
   std::vector<uint16_t *> free_blocks;
   std::vector<RetiredBlock> retired_blocks;
-  uint32_t *scratch = nullptr;  // global work rows for the decode of very wide codes
-  size_t scratch_bytes = 0;
-  // Launches that use `scratch` are ordered across streams by this event:
-  // each waits for the previous user's record, then records its own.
-  cudaEvent_t scratch_done = nullptr;
-  std::mutex scratch_mu;
+  // Global work rows of the register-stage kernels for very wide codes, and the
+  // rows that pass between the bit-sliced GF(2^16) kernels.  Two buffers,
+  // because a launch under stream capture (register-stage kernels) keeps its
+  // pointer in the graph and cannot wait for an event recorded outside it: the
+  // graph's replays may run beside bit-sliced launches on other streams.
+  Slab work, rows16;
   std::vector<uint8_t> dense_enc;  // GF(2^8): the encode map as an m x k matrix
   uint32_t *d_dense_enc = nullptr;  // ... packed for K1, device-resident (filled with dense_enc)
   // GF(2^8) decode maps by (presence pattern, goal), with their K1 tables,
@@ -472,10 +487,7 @@ struct LeopardState {
   ~LeopardState() {
     cudaDeviceSynchronize();
     for (void *p : plan_slabs) cudaFree(p);
-    if (scratch) cudaFreeAsync(scratch, cudaStreamPerThread);  // back to the library's pool
-    for (void *p : owned) cudaFreeAsync(p, cudaStreamPerThread);
     if (d_dense_enc) cudaFree(d_dense_enc);
-    if (scratch_done) cudaEventDestroy(scratch_done);
   }
 };
 
@@ -489,9 +501,10 @@ struct LeoLaunch {
   SliceArgs slice{};
   SliceShape slice_shape;
   // Bit-sliced GF(2^16) kernels (leo_slice16.cu), with the rows that pass
-  // between them in own_scratch or scratch16 (the codec's slab when the launch
+  // between them in own_scratch or scratch16 (the codec's rows16 when the launch
   // was built).  A launch under stream capture runs the engine's kernels
-  // instead: replays could overlap on the slab, and theirs need none (encode).
+  // instead, in shared memory or in the codec's `work`: its replays would
+  // share rows16 with other launches, and nothing would order them.
   bool sliced16 = false;
   Slice16Args slice16{};
   void *scratch16 = nullptr;
@@ -517,25 +530,25 @@ struct LeoLaunch {
   }
 };
 
-// Grow the codec's scratch slab to `need` bytes.  A slab another thread may
-// still have in a built launch is retired (kept until the codec is
-// destroyed), never freed under it.  Slabs come from the library's pool, which
-// keeps what a destroyed codec gave back: mapping 256 MiB afresh took 2 ms of a
-// codec's first launch.
-int grow_scratch(LeopardState &st, size_t need) {
-  std::lock_guard<std::mutex> g(st.scratch_mu);
-  if (st.scratch_bytes >= need) return RSGPU_OK;
-  if (st.scratch) st.owned.push_back(st.scratch);
-  st.scratch = nullptr;
-  st.scratch_bytes = 0;
-  RS_CUDA(cudaError_t(lib_malloc_async(&st.scratch, need, cudaStreamPerThread)));
-  const cudaError_t e = cudaStreamSynchronize(cudaStreamPerThread);  // usable on any stream from here
-  if (e != cudaSuccess) {
-    cudaFreeAsync(st.scratch, cudaStreamPerThread);
-    st.scratch = nullptr;
-    return cuda_status(e);
+// Grows a slab to `need` bytes and gives its buffer.  The memory comes from the
+// library's pool, which keeps what a destroyed codec gave back: mapping 256 MiB
+// afresh took 2 ms of a codec's first launch.
+static int grow_slab(Slab &slab, size_t need, void **out) {
+  std::lock_guard<std::mutex> g(slab.mu);
+  if (slab.bytes < need) {
+    if (slab.ptr) slab.retired.push_back(slab.ptr);
+    slab.ptr = nullptr;
+    slab.bytes = 0;
+    RS_CUDA(cudaError_t(lib_malloc_async(&slab.ptr, need, cudaStreamPerThread)));
+    const cudaError_t e = cudaStreamSynchronize(cudaStreamPerThread);  // usable on any stream from here
+    if (e != cudaSuccess) {
+      cudaFreeAsync(slab.ptr, cudaStreamPerThread);
+      slab.ptr = nullptr;
+      return cuda_status(e);
+    }
+    slab.bytes = need;
   }
-  st.scratch_bytes = need;
+  *out = slab.ptr;
   return RSGPU_OK;
 }
 
@@ -706,12 +719,10 @@ int configure_fft(const K kernel, const K2 kernel_wide, LeoLaunch &L, uint32_t r
       L.args.scratch = static_cast<uint32_t *>(L.own_scratch);
       return RSGPU_OK;
     }
-    int rc = grow_scratch(st, need);
+    void *work = nullptr;
+    int rc = grow_slab(st.work, need, &work);
     if (rc) return rc;
-    {
-      std::lock_guard<std::mutex> g(st.scratch_mu);
-      L.args.scratch = st.scratch;
-    }
+    L.args.scratch = static_cast<uint32_t *>(work);
   }
   return RSGPU_OK;
 }
@@ -735,12 +746,10 @@ int configure(const K kernel, LeoLaunch &L, uint32_t lanes, size_t len, uint64_t
     L.smem = 0;
     L.grid = int(std::min<uint64_t>(tiles, uint64_t(2 * sm_count())));
     const size_t need = size_t(L.grid) * lanes * nb * 64;
-    int rc = grow_scratch(st, need);
+    void *work = nullptr;
+    int rc = grow_slab(st.work, need, &work);
     if (rc) return rc;
-    {
-      std::lock_guard<std::mutex> g(st.scratch_mu);
-      L.args.scratch = st.scratch;
-    }
+    L.args.scratch = static_cast<uint32_t *>(work);
   }
   return RSGPU_OK;
 }
@@ -1071,9 +1080,8 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
     if (slice16_configure(op, sa)) {
       if (L.own_scratch) {
         L.sliced16 = true;
-      } else if (grow_scratch(st, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs)) == RSGPU_OK) {
-        std::lock_guard<std::mutex> g(st.scratch_mu);
-        L.scratch16 = st.scratch;
+      } else if (grow_slab(st.rows16, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs),
+                           &L.scratch16) == RSGPU_OK) {
         L.sliced16 = true;
       } else {
         cudaGetLastError();  // no room: the register-stage kernels
@@ -1144,10 +1152,10 @@ namespace {
 int leo_launch_kernel(const LeoLaunch &L, cudaStream_t s);
 }
 
-// Launches that use the codec's shared scratch slab (global work rows) wait
-// for the previous such launch on any stream.  Under stream capture the
-// graph's own dependencies order them instead (an event recorded outside a
-// capture cannot be waited on inside it).
+// Launches that use one of the codec's slabs wait for its previous user on any
+// stream.  Under stream capture the graph's own dependencies order them instead
+// (an event recorded outside a capture cannot be waited on inside it); the
+// register-stage kernels then run, so a replay never touches rows16.
 int leo_launch(const LeoLaunch &L, cudaStream_t s) {
   if (L.args.n_jobs == 0) return RSGPU_OK;
   const int op = L.decode ? RSGPU_OP_RECONSTRUCT : L.verify ? RSGPU_OP_VERIFY : RSGPU_OP_ENCODE;
@@ -1156,13 +1164,13 @@ int leo_launch(const LeoLaunch &L, cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   RS_CUDA(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) return leo_launch_kernel(L, s);
-  LeopardState &st = *L.codec->leo;
-  std::lock_guard<std::mutex> g(st.scratch_mu);
-  if (!st.scratch_done) RS_CUDA(cudaEventCreateWithFlags(&st.scratch_done, cudaEventDisableTiming));
-  RS_CUDA(cudaStreamWaitEvent(s, st.scratch_done, 0));
-  int rc = L.sliced16 ? slice16_launch(op, L.slice16, L.scratch16, s) : leo_launch_kernel(L, s);
-  if (rc) return rc;
-  return cuda_status(cudaEventRecord(st.scratch_done, s));
+  Slab &slab = L.sliced16 ? L.codec->leo->rows16 : L.codec->leo->work;
+  std::lock_guard<std::mutex> g(slab.mu);
+  if (!slab.done) RS_CUDA(cudaEventCreateWithFlags(&slab.done, cudaEventDisableTiming));
+  RS_CUDA(cudaStreamWaitEvent(s, slab.done, 0));
+  const int rc = L.sliced16 ? slice16_launch(op, L.slice16, L.scratch16, s) : leo_launch_kernel(L, s);
+  const cudaError_t e = cudaEventRecord(slab.done, s);  // after an error too: some kernels may be queued
+  return rc ? rc : cuda_status(e);
 }
 
 namespace {
