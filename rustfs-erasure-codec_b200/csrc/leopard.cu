@@ -433,14 +433,13 @@ constexpr size_t kLocatorCacheBytes = size_t(32) << 20;
 constexpr size_t kLocatorCacheMinPlans = 64;
 
 // A device buffer that launches on any stream use in turn: each waits for the
-// previous user's event, then records its own.  An outgrown buffer that a built
-// launch may still use is retired: freed with the codec, never under the launch.
+// previous user's event, then records its own.
 struct Slab {
   std::mutex mu;
   void *ptr = nullptr;
   size_t bytes = 0;
   cudaEvent_t done = nullptr;
-  std::vector<void *> retired;
+  std::vector<void *> retired;  // outgrown buffers whose address a launch keeps
   ~Slab() {  // the codec's launches have finished
     for (void *p : retired) cudaFreeAsync(p, cudaStreamPerThread);  // back to the library's pool
     if (ptr) cudaFreeAsync(ptr, cudaStreamPerThread);
@@ -501,13 +500,12 @@ struct LeoLaunch {
   SliceArgs slice{};
   SliceShape slice_shape;
   // Bit-sliced GF(2^16) kernels (leo_slice16.cu), with the rows that pass
-  // between them in own_scratch or scratch16 (the codec's rows16 when the launch
-  // was built).  A launch under stream capture runs the engine's kernels
+  // between them in own_scratch or the codec's rows16 (large enough once the
+  // launch is built).  A launch under stream capture runs the engine's kernels
   // instead, in shared memory or in the codec's `work`: its replays would
   // share rows16 with other launches, and nothing would order them.
   bool sliced16 = false;
   Slice16Args slice16{};
-  void *scratch16 = nullptr;
   void *d_blob = nullptr;  // jobs | pointers | roles
   // One-shot launches allocate the blob on their stream and free it there
   // after the kernel; prepared launches own it until destroyed.
@@ -530,25 +528,37 @@ struct LeoLaunch {
   }
 };
 
-// Grows a slab to `need` bytes and gives its buffer.  The memory comes from the
-// library's pool, which keeps what a destroyed codec gave back: mapping 256 MiB
-// afresh took 2 ms of a codec's first launch.
-static int grow_slab(Slab &slab, size_t need, void **out) {
+// Grows a slab to `need` bytes or more: twice what it had, up to `most`, so that
+// launches of rising sizes grow it a few times.  The new buffer comes first; if
+// there is no room for it the slab stays as it was.  With `keep` the caller
+// stores the buffer's address in a launch (and so perhaps in a graph): an
+// outgrown buffer is then freed with the codec, and all of them together are
+// smaller than the slab.  Otherwise launches take the address when they run, and
+// the outgrown buffer is freed behind its last user.
+// The memory comes from the library's pool, which keeps what a destroyed codec
+// gave back: mapping 256 MiB afresh took 2 ms of a codec's first launch.
+static int grow_slab(Slab &slab, size_t need, size_t most, void **keep) {
   std::lock_guard<std::mutex> g(slab.mu);
   if (slab.bytes < need) {
-    if (slab.ptr) slab.retired.push_back(slab.ptr);
-    slab.ptr = nullptr;
-    slab.bytes = 0;
-    RS_CUDA(cudaError_t(lib_malloc_async(&slab.ptr, need, cudaStreamPerThread)));
-    const cudaError_t e = cudaStreamSynchronize(cudaStreamPerThread);  // usable on any stream from here
+    const cudaStream_t s = cudaStreamPerThread;
+    const size_t want = std::max(need, std::min(2 * slab.bytes, most));
+    void *p = nullptr;
+    RS_CUDA(cudaError_t(lib_malloc_async(&p, want, s)));
+    const cudaError_t e = cudaStreamSynchronize(s);  // usable on any stream from here
     if (e != cudaSuccess) {
-      cudaFreeAsync(slab.ptr, cudaStreamPerThread);
-      slab.ptr = nullptr;
+      cudaFreeAsync(p, s);
       return cuda_status(e);
     }
-    slab.bytes = need;
+    if (slab.ptr && keep) {
+      slab.retired.push_back(slab.ptr);
+    } else if (slab.ptr) {
+      if (slab.done) cudaStreamWaitEvent(s, slab.done, 0);
+      cudaFreeAsync(slab.ptr, s);
+    }
+    slab.ptr = p;
+    slab.bytes = want;
   }
-  *out = slab.ptr;
+  if (keep) *keep = slab.ptr;
   return RSGPU_OK;
 }
 
@@ -714,13 +724,13 @@ int configure_fft(const K kernel, const K2 kernel_wide, LeoLaunch &L, uint32_t r
     L.smem = 0;
     L.threads = kWideThreads;
     L.grid = int(std::min<uint64_t>(tiles, uint64_t(kGlobalBlocks) * sm_count()));
-    const size_t need = size_t(L.grid) * rows * nb * 64;
+    const size_t per_cta = size_t(rows) * nb * 64;
     if (L.own_scratch) {  // sized by the caller for a full grid
       L.args.scratch = static_cast<uint32_t *>(L.own_scratch);
       return RSGPU_OK;
     }
     void *work = nullptr;
-    int rc = grow_slab(st.work, need, &work);
+    int rc = grow_slab(st.work, size_t(L.grid) * per_cta, size_t(kGlobalBlocks) * sm_count() * per_cta, &work);
     if (rc) return rc;
     L.args.scratch = static_cast<uint32_t *>(work);
   }
@@ -745,9 +755,9 @@ int configure(const K kernel, LeoLaunch &L, uint32_t lanes, size_t len, uint64_t
     // Work rows in a device slab: one region per resident CTA.
     L.smem = 0;
     L.grid = int(std::min<uint64_t>(tiles, uint64_t(2 * sm_count())));
-    const size_t need = size_t(L.grid) * lanes * nb * 64;
+    const size_t per_cta = size_t(lanes) * nb * 64;
     void *work = nullptr;
-    int rc = grow_slab(st.work, need, &work);
+    int rc = grow_slab(st.work, size_t(L.grid) * per_cta, size_t(2 * sm_count()) * per_cta, &work);
     if (rc) return rc;
     L.args.scratch = static_cast<uint32_t *>(work);
   }
@@ -1081,7 +1091,7 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
       if (L.own_scratch) {
         L.sliced16 = true;
       } else if (grow_slab(st.rows16, slice16_scratch_bytes(sa, uint64_t(sa.tiles_per_job) * sa.n_jobs),
-                           &L.scratch16) == RSGPU_OK) {
+                           kSlabScratch16, nullptr) == RSGPU_OK) {
         L.sliced16 = true;
       } else {
         cudaGetLastError();  // no room: the register-stage kernels
@@ -1168,7 +1178,7 @@ int leo_launch(const LeoLaunch &L, cudaStream_t s) {
   std::lock_guard<std::mutex> g(slab.mu);
   if (!slab.done) RS_CUDA(cudaEventCreateWithFlags(&slab.done, cudaEventDisableTiming));
   RS_CUDA(cudaStreamWaitEvent(s, slab.done, 0));
-  const int rc = L.sliced16 ? slice16_launch(op, L.slice16, L.scratch16, s) : leo_launch_kernel(L, s);
+  const int rc = L.sliced16 ? slice16_launch(op, L.slice16, slab.ptr, s) : leo_launch_kernel(L, s);
   const cudaError_t e = cudaEventRecord(slab.done, s);  // after an error too: some kernels may be queued
   return rc ? rc : cuda_status(e);
 }

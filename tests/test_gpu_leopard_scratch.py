@@ -98,3 +98,79 @@ def test_rebuild_captured_after_one_plain_launch(k, m):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(buf, want)
+
+
+@pytest.mark.parametrize("shift,step,count,bound", [
+    (0, 2048, 41, 3 << 30),    # bit-sliced rows: 6 MiB more a step; the library's pool keeps 2 GiB of freed memory
+    (4, 128, 148, 512 << 20),  # shards off 16 bytes: work rows of one more CTA a step
+])
+def test_rebuilds_of_rising_sizes_hold_a_bounded_amount(shift, step, count, bound):
+    import torch
+
+    import rsgpu
+
+    k, m = 1024, 512
+    codec = _codec(k, m)
+    buf = torch.zeros((k + m) * step * (count + 1) + 16, dtype=torch.uint8, device="cuda")
+    pres = np.ones((1, k + m), np.uint8)
+    pres[0, :8] = 0
+    free = None
+    for i in range(count):
+        length = step * (i + 1)
+        ptrs = rsgpu.device_pointer_table(buf.data_ptr() + shift,
+                                          np.arange(k + m, dtype=np.uint64) * np.uint64(length))
+        codec.prepare_batch("reconstruct", ptrs, length, present=pres).launch()
+        torch.cuda.synchronize()
+        if free is None:
+            free = torch.cuda.mem_get_info()[0]
+    assert free - torch.cuda.mem_get_info()[0] < bound
+
+
+_NO_ROOM = """
+import numpy as np, torch, rsgpu
+k, m, length, stripes = 512, 256, 16384, 16
+codec = rsgpu.ReedSolomon(k, m, rsgpu.CodecOptions(codec_family="leopard_gf16"))
+want = torch.randint(0, 256, (stripes, k + m, length), dtype=torch.uint8, device="cuda")
+for stripe in range(stripes):  # one by one, in little scratch
+    codec.encode_batch(want[stripe:stripe + 1])
+buf = want.clone()
+offsets = np.arange(stripes * (k + m), dtype=np.uint64) * np.uint64(length)
+pres = np.ones((stripes, k + m), np.uint8)
+pres[:, :m] = 0
+def rebuild(n):
+    batch = codec.prepare_batch("reconstruct", rsgpu.device_pointer_table(buf.data_ptr(), offsets[:n * (k + m)]), length,
+                                present=pres[:n])
+    buf[:n, :m] = 0
+    batch.launch()
+    torch.cuda.synchronize()
+    assert torch.equal(buf, want)
+    return batch
+# Every kernel of the path loads while there is memory for its code.
+odd = torch.zeros((k + m) * 64 + 16, dtype=torch.uint8, device="cuda")
+codec.prepare_batch("reconstruct", rsgpu.device_pointer_table(odd.data_ptr() + 4, np.arange(k + m, dtype=np.uint64) *
+                    np.uint64(64)), 64, present=pres[:1]).launch()
+small = rebuild(2)
+assert small.kernel_count() == 3
+torch.cuda.synchronize()
+full = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+for n in (stripes, 2, stripes):
+    assert rebuild(n).kernel_count() == (3 if n == 2 else 1), n
+buf[:2, :m] = 0
+small.launch()
+torch.cuda.synchronize()
+assert torch.equal(buf, want)
+print("done")
+"""
+
+
+def test_no_room_for_larger_rows_leaves_the_smaller_ones_in_use():
+    """In a process of its own: the library's pool holds nothing else there."""
+    import os
+    import subprocess
+    import sys
+
+    import rsgpu
+
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(rsgpu.__file__)))
+    done = subprocess.run([sys.executable, "-c", _NO_ROOM], env=env, capture_output=True, text=True, timeout=300)
+    assert done.stdout.strip().endswith("done"), done.stderr[-2000:]
