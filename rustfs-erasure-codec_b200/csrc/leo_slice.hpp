@@ -44,6 +44,10 @@ void slice_elements(int bits, const uint16_t *exp, uint32_t order, uint16_t *out
 // 1391 us with 96 MiB, 1302 with 256, 1161 with 900 (every tile at once),
 // encodes in 567, 556 and 523.
 constexpr uint64_t kSlabScratch16 = uint64_t(256) << 20, kStreamScratch16 = uint64_t(96) << 20;
+// Launches that need up to this have rows of their own instead: about where a
+// launch fills the GPU by itself (1024+512 encode of one 16 KiB stripe, 25 MiB),
+// so that larger ones lose nothing by running one after another.
+constexpr uint64_t kOwnRows16 = uint64_t(32) << 20;
 // GF(2^16).  Fills the split and tile counts of `a` (its geometry, len, n_jobs
 // and max_scratch set); false when the code or shard length is not covered.
 bool slice16_configure(int op, Slice16Args &a);

@@ -174,3 +174,57 @@ def test_no_room_for_larger_rows_leaves_the_smaller_ones_in_use():
     env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(rsgpu.__file__)))
     done = subprocess.run([sys.executable, "-c", _NO_ROOM], env=env, capture_output=True, text=True, timeout=300)
     assert done.stdout.strip().endswith("done"), done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("op,prepared", [("encode", True), ("verify", True), ("reconstruct", True),
+                                         ("encode", False), ("reconstruct", False)])
+def test_launches_of_one_codec_do_not_wait_for_another_stream(op, prepared):
+    """A small launch finishes while one of the same codec is held up behind
+    other work on its own stream (at most 1 second of it)."""
+    import torch
+
+    k, m, length, stripes = 200, 60, 4096, 2
+    codec = _codec(k, m)
+    want = torch.from_numpy(_codewords(k, m, length, stripes, 9)).cuda()
+    pres = np.ones((stripes, k + m), np.uint8)
+    pres[:, 3:3 + m] = 0
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    bufs = [want.clone() for _ in streams]
+    batches = [codec.prepare_batch(op, _pointers(b), length, present=pres if op == "reconstruct" else None) for b in bufs]
+
+    def wipe(buf):
+        if op == "encode":
+            buf[:, k:] = 0
+        elif op == "reconstruct":
+            buf[:, 3:3 + m] = 0
+
+    def launch(i):
+        with torch.cuda.stream(streams[i]):
+            if prepared:
+                batches[i].launch()
+            elif op == "encode":
+                codec.encode_batch(bufs[i])
+            else:
+                codec.reconstruct_batch(bufs[i], pres)
+
+    for i in range(2):  # every kernel is loaded
+        launch(i)
+    torch.cuda.synchronize()
+    for b in bufs:
+        wipe(b)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(500_000_000)  # a quarter of a second
+        held = torch.cuda.Event()
+        launch(0)
+        held.record()
+    launch(1)
+    streams[1].synchronize()
+    assert not held.query()
+    assert torch.equal(bufs[1], want)
+    torch.cuda.synchronize()
+    assert torch.equal(bufs[0], want)
+    if op == "verify":
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                assert batches[i].verify_result().all()
