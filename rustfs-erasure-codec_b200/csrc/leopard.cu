@@ -432,6 +432,18 @@ struct RetiredBlock {
 constexpr size_t kLocatorCacheBytes = size_t(32) << 20;
 constexpr size_t kLocatorCacheMinPlans = 64;
 
+// Makes `device` current, and the one before it again at the end.
+struct DeviceScope {
+  int prev = -1;
+  explicit DeviceScope(int device) {
+    int cur = 0;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != device && cudaSetDevice(device) == cudaSuccess) prev = cur;
+  }
+  ~DeviceScope() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
 // A device buffer that launches on any stream use in turn: each waits for the
 // previous user's event, then records its own.  Or the buffer of one launch
 // that runs once, on `stream` (`ordered`): no event, freed behind it there.
@@ -443,7 +455,9 @@ struct Slab {
   std::vector<void *> retired;  // outgrown buffers whose address a launch keeps
   bool ordered = false;
   cudaStream_t stream = nullptr;
+  int device = 0;  // of the buffers: cudaStreamPerThread is a stream of the current device
   ~Slab() {
+    DeviceScope scope(device);
     const cudaStream_t s = ordered ? stream : cudaStreamPerThread;
     if (done) cudaStreamWaitEvent(s, done, 0);  // the last user
     for (void *p : retired) cudaFreeAsync(p, s);  // back to the library's pool
@@ -488,7 +502,9 @@ struct LeopardState {
   // Bytes reconstructed so far under patterns whose map is not derived yet
   // (bounded: cleared when it holds kDenseSeenMax patterns).
   std::unordered_map<std::string, size_t> dense_seen;
+  int device = 0;
   ~LeopardState() {
+    DeviceScope scope(device);  // whichever is current where the codec is destroyed
     cudaDeviceSynchronize();
     for (void *p : plan_slabs) cudaFree(p);
     if (d_dense_enc) cudaFree(d_dense_enc);
@@ -552,6 +568,7 @@ static int grow_slab(Slab &slab, size_t need, size_t most, void **keep) {
     const cudaStream_t s = slab.ordered ? slab.stream : cudaStreamPerThread;
     const size_t want = std::max(need, std::min(2 * slab.bytes, most));
     void *p = nullptr;
+    RS_CUDA(cudaGetDevice(&slab.device));
     RS_CUDA(cudaError_t(lib_malloc_async(&p, want, s)));
     const cudaError_t e = slab.ordered ? cudaSuccess : cudaStreamSynchronize(s);  // usable on any stream from here
     if (e != cudaSuccess) {
@@ -574,6 +591,7 @@ static int grow_slab(Slab &slab, size_t need, size_t most, void **keep) {
 int Codec::init_leopard() {
   RS_CUDA(cudaGetDevice(&device));
   auto st = std::make_shared<LeopardState>();
+  st->device = device;
   int rc = leo_field(family == RSGPU_FAMILY_LEOPARD_GF8 ? 8 : 16, &st->field);
   if (rc) return rc;
   st->m = uint32_t(pow2_at_least(m));

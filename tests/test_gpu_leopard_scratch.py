@@ -228,3 +228,31 @@ def test_launches_of_one_codec_do_not_wait_for_another_stream(op, prepared):
         for i in range(2):
             with torch.cuda.stream(streams[i]):
                 assert batches[i].verify_result().all()
+
+
+def test_codec_destroyed_while_another_device_is_current():
+    """Its buffers go back only behind its last kernels."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    k, m, length, stripes = 512, 256, 16384, 8
+    want = torch.from_numpy(_codewords(k, m, length, 2, 3)).cuda().repeat(stripes // 2, 1, 1).contiguous()
+    pres = np.ones((stripes, k + m), np.uint8)
+    pres[:, :m] = 0
+    bufs = [want.clone() for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for b in bufs:
+        b[:, :m] = 0
+    torch.cuda.synchronize()
+    for i, b in enumerate(bufs):  # the second would work in the first one's rows
+        codec = _codec(k, m)
+        with torch.cuda.stream(streams[i]):
+            if i == 0:
+                torch.cuda._sleep(500_000_000)
+            codec.reconstruct_batch(b, pres)
+        with torch.cuda.device(1):
+            del codec
+    torch.cuda.synchronize()
+    for b in bufs:
+        assert torch.equal(b, want)
