@@ -94,12 +94,6 @@ SliceKernel slice_kernel(int op, uint32_t wt) {
 
 }  // namespace
 
-bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t columns) {
-  if (op == RSGPU_OP_RECONSTRUCT) return n > 8 || columns >= (512 << 10);
-  if (m > 16) return true;
-  return k <= 4 * m && (m == 16 || columns >= (2 << 20));
-}
-
 namespace {
 // Rows, threads a row and shared memory of a tile.
 void slice_tile(int op, SliceArgs &a, SliceShape &sh) {

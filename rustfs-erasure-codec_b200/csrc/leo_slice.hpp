@@ -6,6 +6,7 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "leo_rules.hpp"
 #include "leo_types.hpp"
 
 namespace rsgpu {
@@ -14,21 +15,6 @@ struct SliceShape {
   int grid = 0, threads = 0;
   size_t smem = 0;
 };
-// Whether operation op (RSGPU_OP_*) of a code (m, n: transform sizes) over
-// `columns` byte columns in all is faster here than in the register-stage
-// kernels (leo_fft.cuh).  Their work rows in shared memory (m > 16, decode n
-// > 16) always lose to the sliced kernels.  Transforms that fit a thread's
-// registers there have no such passes and use 4 columns a thread instead of
-// 32, so they win on little work, and their data groups need no barriers, so
-// they win when k is many times m.  One B200, register-stage / sliced, us:
-//   encode 10+4   1 MiB columns 9.9 / 10.1,  2 MiB 15.8 / 13.6, 8 MiB 66 / 47
-//   encode 4+2    1 MiB 4.9 / 5.5,           2 MiB 7.4 / 6.5
-//   encode 60+2   2 MiB 62.3 / 61.9;  100+1  2 MiB 44 / 72
-//   encode 32+16  256 KiB 12.9 / 11.8,       8 MiB 246 / 170
-//   rebuild 4+2   256 KiB 6.7 / 7.5,         512 KiB 8.1 / 7.7
-//   rebuild 10+4  256 KiB 13.7 / 11.5,       8 MiB 227 / 87
-//   rebuild 128+64  1 MiB 1068 / 279, encode 246 / 122
-bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t columns);
 // Fills the tile width and rows of `a` (its geometry, len and n_jobs set) and
 // the launch shape of operation op (RSGPU_OP_*).
 int slice_configure(int op, SliceArgs &a, SliceShape &sh);

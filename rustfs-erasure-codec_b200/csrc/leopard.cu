@@ -1138,7 +1138,7 @@ int build_leo(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const 
     }
   }
   if (L.engine == 1 && st.field->bits == 8) {
-    if ((low & 15) == 0 && (lens || slice_pays(op, a.k, a.m, a.n, uint64_t(len) * a.n_jobs))) {
+    if ((low & 15) == 0 && (lens || slice_pays(op, a.k, a.m, a.n, len, uint64_t(len) * a.n_jobs))) {
       L.engine = 2;
       SliceArgs &sa = L.slice;
       sa.jobs = a.jobs;
@@ -1354,7 +1354,10 @@ int prepare_leo_sliced(Codec &c, int op, size_t n, uint8_t *const *shards, const
 
 bool leo_slice_takes(Codec &c, int op, uint64_t columns) {
   const LeopardState &st = *c.leo;
-  return st.field->bits == 8 && leo_engine() == 1 && slice_pays(op, uint32_t(c.k), st.m, st.n, columns);
+  if (st.field->bits != 8 || leo_engine() != 1) return false;
+  // k_mix runs these transforms slower than launches of their own would.
+  if (op != RSGPU_OP_RECONSTRUCT && st.m >= 16) return st.m > 16 || c.k <= 64;
+  return slice_pays(op, uint32_t(c.k), st.m, st.n, columns, columns);
 }
 
 static int run_once(Codec &c, int op, size_t n, uint8_t *const *shards, const uint8_t *present, size_t len, int goal,

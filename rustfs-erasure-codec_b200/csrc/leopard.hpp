@@ -42,7 +42,10 @@ size_t leo_reconstruct_scratch_bytes(Codec &c);
 int prepare_leo_sliced(Codec &c, int op, size_t n, uint8_t *const *shards, const uint8_t *present, const size_t *lens,
                        int goal, const uint32_t *flag_of, uint32_t *flags, cudaStream_t s, bool one_shot,
                        std::shared_ptr<LeoLaunch> &out);
-// Whether those kernels are the faster ones for this much work in all.
+// Whether those kernels are the faster ones for a mixed batch's work of one
+// codec and operation (256 KiB of columns and more; one B200, in k_mix / in a
+// launch of their own: encode 32+16 256 KiB 18 / 14 us, 1 MiB 38 / 29; 60+20
+// 256 KiB 48 / 19; 128+64 256 KiB 92 / 45).
 bool leo_slice_takes(Codec &c, int op, uint64_t columns);
 void leo_set_scratch(LeoLaunch &l, void *scratch);
 int prepare_tower(Codec &c, int op, size_t n_stripes, uint8_t *const *shards, const uint8_t *present, size_t len,
