@@ -35,4 +35,32 @@ inline bool slice_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t len,
   return len >= 512 && (columns >= (56u << 10) || (verify && m == 64 && k <= 128));
 }
 
+// GF(2^16): the same for n_jobs stripes.  These kernels need 64 lanes to split
+// and work on tiles of 2 KiB of a shard, which a length like 2112 fills to
+// half; three launches a pass cost them some 20 us.  The register-stage kernels
+// take one wave of 148 tiles of 128 to 512 bytes in about the time of one
+// tile, and an encode's data groups one after another.  So encodes and verifies
+// of few lanes go there up to one wave of columns (a single data group: two),
+// and from four groups on only when the tiles are badly filled; the widest
+// never.  One B200, register-stage / bit-sliced, us, a launch among others:
+//   encode 60+64   64 KiB 17 / 24, 128 KiB 25 / 25, 256 KiB 45 / 33
+//   encode 120+64  64 KiB 23 / 25, 128 KiB 35 / 29;  180+64 32 KiB 25 / 25 (verify 29 / 31), 128 KiB 47 / 37
+//   encode 200+60  2 KiB 29 / 25, 2112 bytes x 64 55 / 61
+//   encode 100+128 32 KiB 19 / 25, 64 KiB 27 / 27, 128 KiB 51 / 33
+//   encode 200+128 32 KiB 25 / 26, 64 KiB 39 / 31, 2112 bytes x 32 39 / 45
+//   encode 256+256 16 KiB 21 / 25, 32 KiB 39 / 29;  400+200 1 KiB x 4 29 / 27, x 16 29 / 31
+//   encode 500+500 1 KiB 35 / 27, x 16 35 / 38, 2 KiB x 16 68 / 39, 1024+512 1 KiB x 8 51 / 35
+//   encode 2048+1024 1 KiB 117 / 33, 16 KiB x 16 1882 / 858;  1024+512 16 KiB x 16 735 / 360
+//   rebuild 40+16  1 KiB 39 / 23, 64+32 2 KiB x 4 43 / 25, 1024+512 16 KiB x 16 2412 / 1018
+inline bool slice16_pays(int op, uint32_t k, uint32_t m, uint32_t n, uint64_t len, uint64_t n_jobs) {
+  const uint64_t row = 2048, tiles = (len + row - 1) / row * n_jobs, columns = len * n_jobs;
+  if (op == RSGPU_OP_RECONSTRUCT) return n >= 64 && len >= 1024;
+  if (m < 64 || len < (m > 128 ? 1024 : 2048)) return false;
+  if (m >= 1024) return true;
+  const uint32_t groups = (k + m - 1) / m;
+  const uint64_t wave = 148 * (m > 256 ? 128 : 32768 / m);
+  if (m >= 256) return columns > wave || (tiles <= 8 && (groups > 1 || m == 512));
+  return 3 * columns >= 2 * tiles * row && (groups > 3 || columns > (groups == 1 ? 2 : 1) * wave);
+}
+
 }  // namespace rsgpu

@@ -345,15 +345,7 @@ uint32_t log2u(uint32_t v) {
 bool slice16_configure(int op, Slice16Args &a) {
   const bool dec = op == RSGPU_OP_RECONSTRUCT;
   const uint32_t b = log2u(dec ? a.n : a.m);
-  // Where this pays (one B200, register-stage / here, us):
-  //   rebuild 1024+512 16 KiB x 16 2412 / 1018, 300+100 674 / 251, 64+32 118 / 61,
-  //   48+16 (64 lanes) 66 / 40, 40+16 16 KiB x 1 44 / 27, 1 KiB x 32 44 / 30;
-  //   encode 2048+1024 16 KiB x 16 1882 / 858, 1024+512 735 / 360, 60+200 232 / 71,
-  //   512+128 234 / 146, 200+60 (64 lanes) 111 / 67, 16 KiB x 1 33 / 31,
-  //   2 KiB x 16 34 / 30, but 1 KiB x 64 39 / 42 and 512+128 71 / 76.
-  // Below 64 lanes there is too little to split, and a row (2 KiB of a
-  // shard) is half empty at 1 KiB.
-  if (b < 6 || a.len < (dec || b > 7 ? 1024u : 2048u)) return false;
+  if (!slice16_pays(op, a.k, a.m, a.n, a.len, a.n_jobs)) return false;
   a.bl = dec ? std::min(b / 2, b - 4) : std::max(b / 2, b - 5);
   a.bh = b - a.bl;
   if (a.bl > 6 || a.bh > 6) return false;

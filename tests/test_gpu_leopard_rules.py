@@ -50,3 +50,21 @@ def _encode_and_verify(bits, k, m, length, stripes):
 ])
 def test_gf8(k, m, length, stripes):
     _encode_and_verify(8, k, m, length, stripes)
+
+
+@pytest.mark.parametrize("k,m,length,stripes,sliced", [
+    (30, 33, 2048, 75, True), (64, 64, 2048, 74, False),      # 64 lanes, one data group: 148 KiB
+    (120, 64, 4096, 19, True), (190, 64, 2048, 37, False),    # two and three: 74 KiB
+    (200, 60, 2048, 3, True), (193, 50, 4160, 2, True),       # four; the last tile of three a block
+    (200, 60, 2112, 2, False), (200, 60, 1984, 2, False),     # half-filled tiles, short shards
+    (100, 100, 4096, 19, True), (128, 70, 2048, 37, False),   # 128 lanes: 74 KiB
+    (200, 100, 3072, 13, True), (200, 100, 2048, 18, False),  # two groups: 37 KiB, tiles filled to three quarters
+    (512, 128, 2048, 1, True), (300, 128, 2048, 18, False),
+    (256, 256, 1088, 18, True), (60, 200, 1024, 18, False),   # 256 lanes: 18.5 KiB
+    (300, 256, 1024, 8, True), (300, 256, 1024, 9, False),    # two groups: up to 8 tiles too
+    (100, 500, 1024, 8, True), (600, 500, 1088, 9, False), (600, 300, 1088, 18, True),  # 512 lanes
+    (100, 1000, 1024, 9, True),
+])
+def test_gf16(k, m, length, stripes, sliced):
+    batch = _encode_and_verify(16, k, m, length, stripes)
+    assert batch.kernel_count() == (3 if sliced else 1)

@@ -99,7 +99,67 @@ def test_gf8_rule_picks_the_faster_kernels(tmp_path):
     _check(GF8, _picks(tmp_path, "rsgpu::slice_pays(int(op), k, m, n, len, len * stripes)", 8, GF8))
 
 
+GF16 = [
+    (ENCODE, 20, 33, 2048, 1, 14, 19),
+    (ENCODE, 20, 33, 65536, 2, 21, 25),
+    (ENCODE, 60, 64, 65536, 2, 25, 25),
+    (ENCODE, 60, 64, 65536, 4, 45, 33),
+    (ENCODE, 60, 64, 2112, 64, 26, 31),
+    (ENCODE, 120, 64, 4096, 4, 21, 22),
+    (ENCODE, 120, 64, 65536, 1, 23, 25),
+    (ENCODE, 120, 64, 65536, 2, 35, 29),
+    (ENCODE, 120, 64, 2112, 64, 37, 43),
+    (VERIFY, 180, 64, 32768, 1, 29, 31),
+    (ENCODE, 180, 64, 2112, 32, 29, 35),
+    (ENCODE, 180, 64, 2048, 64, 47, 37),
+    (ENCODE, 200, 60, 2048, 1, 29, 25),
+    (ENCODE, 200, 60, 2112, 64, 55, 61),
+    (ENCODE, 200, 60, 16384, 1, 29, 26),
+    (ENCODE, 100, 128, 2048, 1, 17, 21),
+    (ENCODE, 100, 128, 16384, 2, 19, 25),
+    (ENCODE, 100, 128, 65536, 2, 51, 33),
+    (ENCODE, 200, 128, 2048, 16, 25, 26),
+    (ENCODE, 200, 128, 2048, 32, 39, 31),
+    (ENCODE, 200, 128, 2112, 32, 39, 45),
+    (ENCODE, 300, 128, 2112, 16, 31, 37),
+    (ENCODE, 300, 128, 2048, 32, 51, 37),
+    (ENCODE, 100, 200, 1024, 1, 20, 25),
+    (ENCODE, 256, 256, 16384, 1, 21, 25),
+    (ENCODE, 256, 256, 2048, 16, 39, 29),
+    (ENCODE, 400, 200, 1024, 4, 29, 27),
+    (ENCODE, 400, 200, 1024, 16, 29, 31),
+    (ENCODE, 400, 200, 2048, 16, 53, 32),
+    (ENCODE, 600, 256, 2048, 4, 35, 29),
+    (ENCODE, 600, 256, 1024, 64, 131, 100),
+    (ENCODE, 500, 500, 1024, 1, 35, 27),
+    (ENCODE, 500, 500, 1024, 16, 35, 38),
+    (ENCODE, 500, 500, 2048, 16, 68, 39),
+    (ENCODE, 1024, 512, 1024, 8, 51, 35),
+    (ENCODE, 1024, 512, 1088, 16, 52, 58),
+    (ENCODE, 1024, 512, 1024, 32, 101, 96),
+    (ENCODE, 100, 1000, 1024, 16, 61, 54),
+    (ENCODE, 2048, 1024, 1024, 1, 117, 33),
+    (ENCODE, 2048, 1024, 2112, 64, 1071, 838),
+    (VERIFY, 60, 64, 65536, 1, 21, 29),
+    (VERIFY, 60, 64, 65536, 4, 51, 37),
+    (VERIFY, 128, 100, 65536, 1, 31, 33),
+    (VERIFY, 128, 100, 65536, 2, 54, 36),
+    (VERIFY, 256, 256, 1024, 16, 25, 31),
+    (VERIFY, 60, 200, 65536, 1, 76, 35),
+    (VERIFY, 1024, 512, 1024, 16, 55, 61),
+    (VERIFY, 1024, 512, 4096, 1, 55, 33),
+    (RECONSTRUCT, 40, 16, 1024, 1, 39, 23),
+    (RECONSTRUCT, 64, 32, 2048, 4, 43, 25),
+    (RECONSTRUCT, 1024, 512, 1024, 1, 162, 38),
+]
+
+
+def test_gf16_rule_picks_the_faster_kernels(tmp_path):
+    _check(GF16, _picks(tmp_path, "rsgpu::slice16_pays(int(op), k, m, n, len, stripes)", 16, GF16))
+
+
+@pytest.mark.parametrize("cases", [GF8, GF16])
 @pytest.mark.parametrize("sliced", [False, True])
-def test_a_wrong_rule_is_seen(tmp_path, sliced):
+def test_a_wrong_rule_is_seen(cases, sliced):
     with pytest.raises(AssertionError):
-        _check(GF8, [sliced] * len(GF8))
+        _check(cases, [sliced] * len(cases))
