@@ -304,10 +304,21 @@ __device__ __forceinline__ bool apply_column(const uint8_t *const *ptrs, const J
   bool bad = false;
   for (uint32_t g = 0; g * 4 < d.n_out; ++g) {
     uint32_t acc = 0;
-    for (uint32_t j = 0; j < d.n_in; ++j) {
-      const uint32_t x = ptr[j][col];
-      const uint32_t *tb = d.tbl + (g * d.n_in + j) * kTableWords;
-      acc ^= __ldg(tb + (x & 15)) ^ __ldg(tb + 16 + (x >> 4));
+    // One loop in the two forms that compile to the shorter chain of loads:
+    // 50+20 of 5001 bytes, encode 45 us in the first and 35 in the second,
+    // verify 29 and 39.
+    if (VERIFY) {
+      for (uint32_t j = 0; j < d.n_in; ++j) {
+        const uint32_t x = ptr[j][col];
+        const uint32_t *tb = d.tbl + (g * d.n_in + j) * kTableWords;
+        acc ^= __ldg(tb + (x & 15)) ^ __ldg(tb + 16 + (x >> 4));
+      }
+    } else {
+      const uint32_t *tb = d.tbl + size_t(g) * d.n_in * kTableWords;
+      for (uint32_t j = 0; j < d.n_in; ++j, tb += kTableWords) {
+        const uint32_t x = ptr[j][col];
+        acc ^= __ldg(tb + (x & 15)) ^ __ldg(tb + 16 + (x >> 4));
+      }
     }
     for (uint32_t r = 0; r < 4 && g * 4 + r < d.n_out; ++r) {
       uint8_t *dst = const_cast<uint8_t *>(ptr[d.n_in + g * 4 + r]) + col;

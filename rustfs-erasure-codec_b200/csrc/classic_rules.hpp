@@ -1,0 +1,32 @@
+// classic_rules.hpp -- which K1 kernel takes jobs whose shards are not all
+// 16-byte aligned.  Plain host arithmetic, so that a test can compare the rule
+// with measurements.
+#pragma once
+
+#include <cstdint>
+
+namespace rsgpu {
+
+constexpr uint32_t kWordTile = 4096;  // columns of a work item of k_apply_unaligned
+
+// Whether misaligned jobs of len bytes, n_jobs of them with up to max_out
+// outputs, are faster by words (k_apply_unaligned) than one thread a byte
+// column (k_apply_tail).  A word tile takes about as long with few columns as
+// with 4096, and outputs in fours one after another, so the byte kernel wins
+// while it has few columns a thread, and when the tiles are badly filled.  One
+// B200, bytes / words, us:
+//   encode 10+4  312 KiB of columns 10 / 12, 781 KiB 15 / 12, 1.25 MiB 21 / 16
+//   encode 12+4  2.5 MiB in shards of 5001 bytes 41 / 39;  16+4 514 KiB of 1029 14 / 16
+//   encode 10+6  488 KiB 15 / 19, 1.25 MiB 32 / 24
+//   rebuild 50+20 781 KiB 92 / 127, 1.25 MiB 169 / 161, of 5001 bytes 172 / 248
+//   verify 12+4  195 KiB 10 / 12, 312 KiB 12 / 12, 781 KiB 18 / 14
+//   verify 50+20 312 KiB 82 / 119, 781 KiB of 5001 bytes 151 / 208, 1.25 MiB 258 / 208
+inline bool words_pay(bool verify, uint32_t max_out, uint64_t len, uint64_t n_jobs) {
+  const uint64_t words = len >= 12 ? (len - 8) / 4 : 0, columns = len * n_jobs;
+  uint64_t padded = (words * 4 + kWordTile - 1) / kWordTile * kWordTile * n_jobs;
+  if (!words) padded = uint64_t(kWordTile) * n_jobs;
+  if (max_out > 4) return columns >= ((verify ? 512u : 1024u) << 10) && 8 * columns >= 5 * padded;
+  return columns >= ((verify ? 256u : 704u) << 10) && 5 * columns >= 2 * padded;
+}
+
+}  // namespace rsgpu

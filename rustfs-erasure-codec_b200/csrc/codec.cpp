@@ -8,6 +8,8 @@
 #include <map>
 #include <mutex>
 
+#include "classic_rules.hpp"
+
 namespace rsgpu {
 
 static std::atomic<uint64_t> g_launches{0};
@@ -448,10 +450,8 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   max_tail = 0;
   uint32_t max_out = 0, uni_in = jobs.empty() ? 0 : jobs[0].n_in;
   int any_vec = 0, any_unaligned = 0;
-  // Misaligned jobs: by words from about here, one thread a byte column below
-  // (10+4 at 5001 bytes, one stripe: 8 against 13 us; 1029 bytes x 1000: 21
-  // both; 12+4 at 100003 x 128: 351 against 103).
-  const bool words = uint64_t(len) * jobs.size() >= (256u << 10);
+  for (const auto &j : jobs) max_out = std::max<uint32_t>(max_out, j.n_out);
+  const bool words = words_pay(vfy, max_out, len, jobs.size());  // how misaligned jobs go
   int tbl_stage = 0;
   for (auto &j : jobs) {
     tbl_stage |= j.tbl != jobs[0].tbl;
@@ -466,7 +466,6 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
     else
       j.mode |= kJobUnaligned;
     any_unaligned |= !aligned && words;
-    max_out = std::max<uint32_t>(max_out, j.n_out);
     any_vec |= j.vec_len > 0;
   }
   args.flags = flags;

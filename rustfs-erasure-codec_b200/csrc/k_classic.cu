@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include "apply_tile.cuh"
+#include "classic_rules.hpp"
 #include "common.hpp"
 #include "kernels.hpp"
 #include "launch_cfg.hpp"
@@ -439,11 +440,13 @@ __global__ void __launch_bounds__(kApplyThreads + 32, RegShape<K, VERIFY>::kBloc
 }
 
 // Byte-granular path for the columns past each job's vec_len.  One thread per
-// byte column.
-template <bool VERIFY, bool ACC = false>
+// byte column.  INLINE: the job and its pointers are in the arguments; a choice
+// made in the kernel made every read of them a generic one (50+20 encode of
+// 5001-byte shards 37 -> 45 us).
+template <bool VERIFY, bool ACC, bool INLINE>
 __global__ void k_apply_tail(const __grid_constant__ ApplyArgs a, uint64_t max_tail) {
-  const JobDesc *const jobs = job_list(a);
-  const uint8_t *const *const ptrs = ptr_list(a);
+  const JobDesc *const jobs = INLINE ? &a.job : a.jobs;
+  const uint8_t *const *const ptrs = INLINE ? a.job_ptrs : a.ptrs;
   const uint64_t n = max_tail * a.n_jobs;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += uint64_t(gridDim.x) * blockDim.x) {
@@ -464,11 +467,13 @@ __global__ void k_apply_tail(const __grid_constant__ ApplyArgs a, uint64_t max_t
 // most (its neighbour's bytes come by a shuffle) with single bytes at the ends
 // of a warp's run.  The columns covered this way, 4 to 4 + 4 * n, keep every
 // aligned word inside the shard; the few before and after are the work of an
-// extra warp.  The alternative for such jobs was one thread a byte
-// column: verify of 128 12+4 stripes of 100003 bytes
-// 351 -> 103 us, encode 264 -> 115, 24+4 at 50001 bytes x 100 encode 174 -> 77.
+// extra warp.  Against one thread a byte column (k_apply_tail, still the faster
+// one on few columns: classic_rules.hpp): verify of 128 12+4 stripes of 100003
+// bytes 351 -> 103 us, encode 264 -> 115, 24+4 at 50001 bytes x 100 encode
+// 174 -> 77.
 constexpr int kWordsU = 4;
 constexpr uint32_t kTileU = kApplyThreads * 4 * kWordsU;
+static_assert(kTileU == kWordTile, "classic_rules.hpp counts tiles");
 
 // Words of a thread's columns from p on (word v at p + v * kApplyThreads * 4),
 // zero where !on.  Both aligned words are read even when one would do: without
@@ -908,12 +913,11 @@ cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cud
     const uint64_t want = (n + threads - 1) / threads;
     const uint64_t cap = uint64_t(device_sm_count()) * 16;
     const int grid = int(want < cap ? want : cap);
-    if (a.accumulate)
-      k_apply_tail<false, true><<<grid, threads, 0, s>>>(a, max_tail);
-    else if (verify)
-      k_apply_tail<true><<<grid, threads, 0, s>>>(a, max_tail);
-    else
-      k_apply_tail<false><<<grid, threads, 0, s>>>(a, max_tail);
+    auto *fn = a.jobs ? (a.accumulate ? k_apply_tail<false, true, false> : verify ? k_apply_tail<true, false, false>
+                                                                                 : k_apply_tail<false, false, false>)
+                      : (a.accumulate ? k_apply_tail<false, true, true> : verify ? k_apply_tail<true, false, true>
+                                                                                : k_apply_tail<false, false, true>);
+    fn<<<grid, threads, 0, s>>>(a, max_tail);
     ++launches;
   }
   launch_counter_add(launches);
