@@ -1,6 +1,6 @@
-// classic_rules.hpp -- which K1 kernel takes jobs whose shards are not all
-// 16-byte aligned.  Plain host arithmetic, so that a test can compare the rule
-// with measurements.
+// classic_rules.hpp -- which K1 kernel takes misaligned jobs, and verifies of
+// few inputs.  Plain host arithmetic, so that a test can compare the rules with
+// measurements.
 #pragma once
 
 #include <cstdint>
@@ -27,6 +27,17 @@ inline bool words_pay(bool verify, uint32_t max_out, uint64_t len, uint64_t n_jo
   if (!words) padded = uint64_t(kWordTile) * n_jobs;
   if (max_out > 4) return columns >= ((verify ? 512u : 1024u) << 10) && 8 * columns >= 5 * padded;
   return columns >= ((verify ? 256u : 704u) << 10) && 5 * columns >= 2 * padded;
+}
+
+// Whether a verify of n_in inputs a job runs in the staged tile rather than with
+// its tables in registers.  One or two inputs have next to no lookups to share,
+// and the register tile keeps fewer of their bytes on the way (every stage has
+// room for four parity shards).  One B200, staged / in registers, us:
+//   verify 1+1  4 KiB x 1024 12 / 11, 64 KiB x 64 8.4 / 10, 1 MiB x 256 200 / 225
+//   verify 2+1  1 KiB x 1024 14 / 10, 16 KiB x 64 8 / 8, 1 MiB x 64 71 / 75
+//   verify 3+2  1 MiB x 64 90 / 86
+inline bool verify_staged(uint32_t n_in, uint64_t len, uint64_t n_jobs) {
+  return n_in <= 2 && len >= (16u << 10) && len * n_jobs >= (4u << 20);
 }
 
 }  // namespace rsgpu

@@ -296,8 +296,10 @@ struct RegShape {
   // Words a thread reads at a time: two (64-bit reads) while they fit the
   // registers of three CTAs an SM.
   static constexpr int kWords = K <= 10 ? 2 : 1;
-  // Bytes of every shard a tile: enough work between two barrier waits.
-  static constexpr uint32_t kTile = K <= 4 ? 8192 : K <= 7 ? 4096 : 2048;
+  // Bytes of every shard a tile: enough work between two barrier waits.  A
+  // verify of 4 inputs stages 8 shards; at 8 KiB each one CTA would fill the SM
+  // (4+2 1 MiB x 64 121 us; 107 at 4 KiB, as in the staged tile).
+  static constexpr uint32_t kTile = K <= 4 - VERIFY ? 8192 : K <= 7 ? 4096 : 2048;
   static constexpr int kFit = int(74 * 1024 / (kSlots * kTile));
   static constexpr int kStages = kFit < 2 ? 2 : kFit > 4 ? 4 : kFit;
   static constexpr int kBlocks = kFit < 2 || K > 13 ? 2 : 3;
@@ -863,14 +865,15 @@ void launch_unaligned(const ApplyArgs &a, cudaStream_t s) {
 //   encode 4+2    1 MiB x 512 4476 / 5345;  16+4 1 MiB x 256 4209 / 4807
 //   encode 8+4    4 KiB x 4096 2175 / 4278
 //   rebuild 16+4  1 MiB x 256 4109 / 4604;  6+3 256 KiB x 512 4102 / 4765
-//   verify 20+4   1 MiB x 128 4036 / 4231
+//   verify 20+4   1 MiB x 128 4036 / 4231;  of one or two inputs: classic_rules.hpp
 template <bool VERIFY>
 void launch_write_or_verify(const ApplyArgs &a, int variant, cudaStream_t s) {
   if (a.max_out > 4)
     launch_vec<2, 1, VERIFY, false, 2>(a, s);
   else if (variant == 1)
     launch_vec<1, 1, VERIFY, false, 4>(a, s);
-  else if (variant == 0 && a.uni_in >= 1 && a.uni_in <= kRegInputs)
+  else if (variant == 0 && a.uni_in >= 1 && a.uni_in <= kRegInputs &&
+           !(VERIFY && verify_staged(a.uni_in, a.len, a.n_jobs)))
     launch_reg_k<VERIFY>(a, s);
   else
     launch_tma<2, 3, VERIFY>(a, s);

@@ -1,6 +1,7 @@
-"""CPU: the rule that picks a kernel for misaligned classic shards
-(classic_rules.hpp) against times measured on one B200: on either side of its
-lines, the kernel it picks took at most 10% longer than the other."""
+"""CPU: the rules that pick a kernel for misaligned classic shards and for
+verifies of few inputs (classic_rules.hpp) against times measured on one B200: on
+either side of their lines, the kernel they pick took at most 10% longer than the
+other."""
 import pathlib
 import subprocess
 
@@ -39,6 +40,20 @@ TIMES = [
     (VERIFY, 8, 10001, 64, 31, 31),      # 20
 ]
 
+STAGED = 2
+# (, inputs, shard length, stripes, us with tables in registers, us staged)
+FEW_INPUTS = [
+    (STAGED, 1, 1024, 1024, 8, 12),
+    (STAGED, 1, 4096, 1024, 11, 12),
+    (STAGED, 1, 65536, 64, 10.3, 8.4),
+    (STAGED, 1, 1048576, 256, 225, 200),
+    (STAGED, 2, 1024, 1024, 10, 14),
+    (STAGED, 2, 4096, 1024, 12, 15),
+    (STAGED, 2, 1048576, 8, 16.5, 14.5),
+    (STAGED, 3, 262144, 256, 86, 90),
+    (STAGED, 4, 4096, 1024, 15, 20),
+]
+
 _DRIVER = """
 #include <cstdio>
 #include "classic_rules.hpp"
@@ -46,7 +61,7 @@ int main() {
   unsigned verify, outs;
   unsigned long long len, stripes;
   while (scanf("%u %u %llu %llu", &verify, &outs, &len, &stripes) == 4)
-    puts(rsgpu::words_pay(verify, outs, len, stripes) ? "1" : "0");
+    puts((verify == 2 ? rsgpu::verify_staged(outs, len, stripes) : rsgpu::words_pay(verify, outs, len, stripes)) ? "1" : "0");
 }
 """
 
@@ -62,17 +77,19 @@ def _picks(tmp_path, cases):
     return [x == "1" for x in out]
 
 
-def _slow(picks):
-    return [c for c, words in zip(TIMES, picks) if c[5 if words else 4] > 1.1 * min(c[4:])]
+def _slow(cases, picks):
+    return [c for c, second in zip(cases, picks) if c[5 if second else 4] > 1.1 * min(c[4:])]
 
 
-def test_rule_picks_the_faster_kernel(tmp_path):
-    assert not _slow(_picks(tmp_path, TIMES))
+@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS])
+def test_rule_picks_the_faster_kernel(tmp_path, cases):
+    assert not _slow(cases, _picks(tmp_path, cases))
 
 
-@pytest.mark.parametrize("words", [False, True])
-def test_a_wrong_rule_is_seen(words):
-    assert _slow([words] * len(TIMES))
+@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS])
+@pytest.mark.parametrize("second", [False, True])
+def test_a_wrong_rule_is_seen(cases, second):
+    assert _slow(cases, [second] * len(cases))
 
 
 def test_short_shards_and_empty_launches_go_by_bytes(tmp_path):
