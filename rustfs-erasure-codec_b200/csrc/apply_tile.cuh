@@ -180,14 +180,23 @@ struct LutSet {
   }
 };
 
-// Inputs j0 .. j0 + C of one tile and pass: loads, tables and products.
+// Products of C inputs (x: their loaded words) from j0 on.
 template <int C, int NG, int V>
+__device__ __forceinline__ void apply_products(const JobDesc &d, uint32_t g0, uint32_t groups, uint32_t j0,
+                                               const uint4 (*x)[V], uint32_t lane, uint32_t (*acc)[V][16]);
+
+// Inputs j0 .. j0 + C + D of one tile and pass: loads, tables and products.
+// D = 1: one input more that shares no lookups, for what is left of 2 or 4
+// inputs.  Its load is on its way with the others; in a step of its own it made
+// a thread wait for memory once more (k_mix, 4+2 encode of 256 KiB x 64
+// 36.5 -> 33.0 us).
+template <int C, int NG, int V, int D = 0>
 __device__ __forceinline__ void apply_step(const uint8_t *const *ptr, const JobDesc &d, uint32_t g0, uint32_t groups,
                                            uint32_t j0, const uint64_t *col, const bool *active, uint32_t lane,
                                            uint32_t (*acc)[V][16]) {
-  uint4 x[C][V];
+  uint4 x[C + D][V];
 #pragma unroll
-  for (int i = 0; i < C; ++i) {
+  for (int i = 0; i < C + D; ++i) {
     const uint8_t *src = ptr[j0 + i];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
@@ -195,6 +204,13 @@ __device__ __forceinline__ void apply_step(const uint8_t *const *ptr, const JobD
       if (active[v]) x[i][v] = ld_stream(src + col[v]);
     }
   }
+  apply_products<C, NG, V>(d, g0, groups, j0, x, lane, acc);
+  if (D) apply_products<1, NG, V>(d, g0, groups, j0 + C, x + C, lane, acc);
+}
+
+template <int C, int NG, int V>
+__device__ __forceinline__ void apply_products(const JobDesc &d, uint32_t g0, uint32_t groups, uint32_t j0,
+                                               const uint4 (*x)[V], uint32_t lane, uint32_t (*acc)[V][16]) {
   Lut<C> lut[NG];
 #pragma unroll
   for (int g = 0; g < NG; ++g) {
@@ -221,7 +237,8 @@ __device__ __forceinline__ void apply_step(const uint8_t *const *ptr, const JobD
 // kApplyThreads threads of the CTA (warp shuffles need full warps).
 // ACC: outputs accumulate (dst ^= product) instead of being overwritten,
 // for incremental parity updates (encode_single with i > 0, update).
-template <int NG, int V, bool VERIFY, bool ACC = false>
+// FEW: at most 2 inputs.
+template <int NG, int V, bool VERIFY, bool ACC = false, bool FEW = false>
 __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t *flags, const JobDesc &d,
                                            uint64_t tile_base) {
   const uint32_t lane = threadIdx.x & 31;
@@ -247,13 +264,16 @@ __device__ __forceinline__ void apply_tile(const uint8_t *const *ptrs, uint32_t 
         for (int i = 0; i < 16; ++i) acc[g][v][i] = 0;
     uint32_t j = 0;
 #pragma unroll 1
-    for (; j + 5 <= n_in; j += 5) apply_step<5, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
-    if (j + 3 <= n_in) {
+    for (; !FEW && j + 5 <= n_in; j += 5) apply_step<5, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
+    const uint32_t left = n_in - j;  // CTA-uniform
+    if (!FEW && left == 4)
+      apply_step<3, NG, V, 1>(ptr, d, g0, groups, j, col, active, lane, acc);
+    else if (!FEW && left == 3)
       apply_step<3, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
-      j += 3;
-    }
-#pragma unroll 1
-    for (; j < n_in; ++j) apply_step<1, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
+    else if (left == 2)
+      apply_step<1, NG, V, 1>(ptr, d, g0, groups, j, col, active, lane, acc);
+    else if (left == 1)
+      apply_step<1, NG, V>(ptr, d, g0, groups, j, col, active, lane, acc);
     bool bad = false;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
