@@ -33,11 +33,11 @@ __device__ __forceinline__ const uint8_t *const *ptr_list(const ApplyArgs &a) { 
 // Grid-stride loop of apply_tile over every (job, tile) of a launch, inputs
 // loaded straight into registers: the tile for more than 4 outputs and for
 // accumulating (incremental parity) launches.
-template <int NG, int V, bool VERIFY, bool ACC, int MINB>
+template <int NG, bool VERIFY, bool ACC, int MINB>
 __global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(const __grid_constant__ ApplyArgs a) {
   const JobDesc *const jobs = job_list(a);
   const uint8_t *const *const ptrs = ptr_list(a);
-  constexpr uint32_t kTile = kApplyThreads * kApplyVec * V;
+  constexpr uint32_t kTile = kApplyThreads * kApplyVec;
   const uint32_t tiles_per_job = uint32_t((a.len + kTile - 1) / kTile);
   const uint32_t total = tiles_per_job * a.n_jobs;
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -45,12 +45,12 @@ __global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(const __grid_
     const uint64_t tile_base = uint64_t(t - job * tiles_per_job) * kTile;
     const JobDesc d = jobs[job];
     if (tile_base >= d.vec_len) continue;  // CTA-uniform
-    apply_tile<NG, V, VERIFY, ACC>(ptrs, a.flags, d, tile_base);
+    apply_tile<NG, 1, VERIFY, ACC>(ptrs, a.flags, d, tile_base);
   }
 }
 
 // ------------------------------------------------------------------ K1, TMA-staged
-// The same product as k_apply_vec<1, V, 4, 0> with the input tiles staged in
+// The product for at most 4 outputs with the input tiles staged in
 // shared memory by the bulk-copy (TMA) unit: one producer warp streams each
 // step's tile slices (one contiguous 256 * 16 * V-byte slice per input shard,
 // cp.async.bulk with completion on the stage's mbarrier) into a ring of S
@@ -61,8 +61,8 @@ __global__ void __launch_bounds__(kApplyThreads, MINB) k_apply_vec(const __grid_
 // that runs out sets *a.stall (the codec's status word, read back by the
 // next synchronous call as RSGPU_ERR_DEVICE_TIMEOUT), and the producer then
 // waits, bounded again, for the copies it has in flight before it exits.
-// Measured against the register-path tile (k_apply_vec<1, 2, 4, 0>) on
-// 1024 x 1 MiB stripes: 10+4 encode 4650 vs 4268 GB/s; global-load stalls per
+// Measured against inputs loaded straight to registers (32 bytes a thread, four
+// inputs in flight, the same pairs of 16-entry lookups) on 1024 x 1 MiB stripes: 10+4 encode 4650 vs 4268 GB/s; global-load stalls per
 // issued instruction fall from 4.1 to 1.7, and the bulk copies do not compete
 // with the table shuffles for the L1 data pipe (cp.async staging, which
 // does, was 7-14% slower than the register path).
@@ -282,7 +282,8 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(const __gri
 // the data read.  The staged tile above needs 8 shuffles and re-reads two
 // tables per input and step, in 96 registers; this one fits 72, so three CTAs
 // share an SM and the shuffle latency is hidden (10+4 encode, 1 MiB x 512:
-// 4498 -> 5351 GB/s, 83% of the copy peak; the pipe is 81% busy).
+// 4498 -> 5351 GB/s while the clock is at its maximum, the pipe 81% busy; in
+// long runs under the power cap 4083 -> 4637, 72% of the copy peak).
 // A CTA takes a contiguous run of tiles: launches whose stripes carry
 // different tables then change tables once per stripe, not once per tile.
 // The producer warp, the mbarrier ring and its bounded waits are
@@ -796,15 +797,15 @@ int grid_for(const void *fn, int threads, size_t smem) {
   return sms * per_sm;
 }
 
-template <int NG, int V, bool VERIFY, bool ACC, int MINB>
+template <int NG, bool VERIFY, bool ACC, int MINB>
 void launch_vec(const ApplyArgs &a, cudaStream_t s) {
   static int grid_max = 0;
-  const void *fn = (const void *)k_apply_vec<NG, V, VERIFY, ACC, MINB>;
+  const void *fn = (const void *)k_apply_vec<NG, VERIFY, ACC, MINB>;
   if (!grid_max) grid_max = grid_for(fn, kApplyThreads, 0);
-  const uint64_t tile = uint64_t(kApplyThreads) * kApplyVec * V;
+  const uint64_t tile = uint64_t(kApplyThreads) * kApplyVec;
   const uint64_t tiles = ((a.len + tile - 1) / tile) * a.n_jobs;
   const int grid = int(tiles < uint64_t(grid_max) ? tiles : grid_max);
-  k_apply_vec<NG, V, VERIFY, ACC, MINB><<<grid, kApplyThreads, 0, s>>>(a);
+  k_apply_vec<NG, VERIFY, ACC, MINB><<<grid, kApplyThreads, 0, s>>>(a);
 }
 
 template <int V, int S, bool VERIFY>
@@ -869,9 +870,9 @@ void launch_unaligned(const ApplyArgs &a, cudaStream_t s) {
 template <bool VERIFY>
 void launch_write_or_verify(const ApplyArgs &a, int variant, cudaStream_t s) {
   if (a.max_out > 4)
-    launch_vec<2, 1, VERIFY, false, 2>(a, s);
+    launch_vec<2, VERIFY, false, 2>(a, s);
   else if (variant == 1)
-    launch_vec<1, 1, VERIFY, false, 4>(a, s);
+    launch_vec<1, VERIFY, false, 4>(a, s);
   else if (variant == 0 && a.uni_in >= 1 && a.uni_in <= kRegInputs &&
            !(VERIFY && verify_staged(a.uni_in, a.len, a.n_jobs)))
     launch_reg_k<VERIFY>(a, s);
@@ -894,7 +895,7 @@ cudaError_t launch_apply(const ApplyArgs &a, bool verify, uint64_t max_tail, cud
   uint64_t launches = 0;
   if (a.any_vec && a.len >= 16) {
     if (a.accumulate)
-      launch_vec<1, 1, false, true, 4>(a, s);
+      launch_vec<1, false, true, 4>(a, s);
     else if (verify)
       launch_write_or_verify<true>(a, apply_variant(), s);
     else

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(512, 1) k_slice16_a(Slice16Args a) {
             uint32_t y[16];
             cols.load(reinterpret_cast<const uint8_t *>(lane.ptr), y);
             Cols16::planes(y);
-            mac16<4>(lane.c, x, y);
+            mac16(lane.c, x, y);
           }
           row16_store(sbase + (i0 + i) * kRow16, x);
         }
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(512, 1) k_slice16_a(Slice16Args a) {
       __syncthreads();
     }
     const DataRows in{a, jd, R, cols};
-    ifft16<3>(sbase, DEC ? nullptr : &in, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, a.bl, DEC ? R : a.m + R,
+    ifft16(sbase, DEC ? nullptr : &in, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, a.bl, DEC ? R : a.m + R,
               limit - R);
   }
 }
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(512, 1) k_slice16_c(Slice16Args a) {
     const ScratchRows uin{a.u + (size_t(w.x) * a.u_rows + R) * 128 + t};
     const bool derive = MODE == 2 && R < jd.input_count;  // CTA-uniform; past it V is zero
     if (derive) derivative16(sbase, rows, a.v + (size_t(w.x) * a.v_rows + R) * 128 + t, uin.p);
-    fft16<3>(sbase, derive ? nullptr : &uin, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
+    fft16(sbase, derive ? nullptr : &uin, a.bl, R, (MODE == 2 ? a.m + a.k : a.p) - R, need);
     const Cols16 cols(w.col, t, a.len);
     uint32_t bad = 0;
 #pragma unroll 1
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(512, 1) k_slice16_c(Slice16Args a) {
         row16_load(sbase + (i0 + i) * kRow16, v);
         if (MODE == 2) {
           uint32_t x[16] = {};
-          mac16<4>(lane.c, x, v);
+          mac16(lane.c, x, v);
           Cols16::bytes(x);
           cols.store(out, x);
         } else {

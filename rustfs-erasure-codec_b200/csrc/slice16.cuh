@@ -6,8 +6,8 @@
 // and a transform over 2^b lanes is split in two levels, as a large FFT is:
 // 2^bl consecutive lanes (the low layers) and 2^bh lanes 2^bl apart (the high
 // layers), each level a tile of rows in shared memory.  Between the levels the
-// rows pass through a scratch buffer in plane form, sized so that a chunk of
-// tiles stays in L2.
+// rows pass through a scratch buffer in plane form, a chunk of tiles at a time
+// (how many: leo_slice.hpp).
 //
 //   encode:  low IFFT of every data group (A) -> V; per residue, high IFFT of
 //            every group, their XOR, high FFT (B) -> U; low FFT (C) -> parity
@@ -41,19 +41,18 @@ namespace {
 
 constexpr uint32_t kRow16 = 2048;  // bytes of a row: 4 quarters of 16 bytes a thread
 
-template <int NQ>
+// x ^= c * y for a constant of three nibbles (two pairs), and of four.
 __device__ __forceinline__ void mac16x2(uint32_t c, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
                                         const uint32_t *y1) {
   mac2_nibble<16, 0>(c & 15, x0, y0, x1, y1);
   mac2_nibble<16, 4>((c >> 4) & 15, x0, y0, x1, y1);
-  if (NQ > 2) mac2_nibble<16, 8>((c >> 8) & 15, x0, y0, x1, y1);
+  mac2_nibble<16, 8>((c >> 8) & 15, x0, y0, x1, y1);
 }
-template <int NQ>
 __device__ __forceinline__ void mac16(uint32_t c, uint32_t *x, const uint32_t *y) {
   mac_nibble<16, 0>(c & 15, x, y);
   mac_nibble<16, 4>((c >> 4) & 15, x, y);
-  if (NQ > 2) mac_nibble<16, 8>((c >> 8) & 15, x, y);
-  if (NQ > 3) mac_nibble<16, 12>(c >> 12, x, y);
+  mac_nibble<16, 8>((c >> 8) & 15, x, y);
+  mac_nibble<16, 12>(c >> 12, x, y);
 }
 
 // Rows in shared memory; base: this thread's words of row 0.
@@ -101,11 +100,12 @@ __device__ __forceinline__ void zero_row(uint32_t addr) {
 // on rows l, l + d, l + 2d, l + 3d, or with !pair the outer layer alone
 // (distance 2^lgd >= 2) on rows l, l + 1 and their partners.  Positions: row i
 // stands at off + i; where not null, `in` gives the rows (an IFFT's skipped ones
-// are zero) and `out` (this thread's scratch rows) takes them; a group starting at or past `limit` rows is skipped, and
-// so is one with no 4-row block in `need`.  Both layers go through one copy of
-// the networks (the loop below), with the middle rows exchanged in between:
-// two copies, 34 KB each, overflowed the instruction cache.
-template <int NQ, bool FWD, class In>
+// are zero) and `out` (this thread's scratch rows) takes them; a group starting
+// at or past `limit` rows is skipped, and so is one with no 4-row block in
+// `need`.  Both layers go through one copy of the networks (the loop below), with
+// the middle rows exchanged in between: two copies, 34 KB each, overflowed the
+// instruction cache.
+template <bool FWD, class In>
 __device__ __forceinline__ void pass16(uint32_t s, const In *in, uint4 *out, uint32_t rows, uint32_t lgd, bool pair,
                                        uint32_t off, uint32_t limit, uint32_t need) {
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void pass16(uint32_t s, const In *in, uint4 *out, uin
         xor_planes<16>(v[1], v[0]);
         xor_planes<16>(v[3], v[2]);
       }
-      mac16x2<NQ>(inner ? e_in : e_out, v[0], v[1], v[2], v[3]);
+      mac16x2(inner ? e_in : e_out, v[0], v[1], v[2], v[3]);
       if (inner) mac_const<16, 2>(v[2], v[3]);
       if (FWD) {
         xor_planes<16>(v[1], v[0]);
@@ -174,26 +174,25 @@ __device__ __forceinline__ void pass16(uint32_t s, const In *in, uint4 *out, uin
 }
 // IFFT over 2^b rows (b >= 3); the first pass reads `in`, unless null, the
 // last one writes out, shared memory is in between.
-template <int NQ, class In>
+template <class In>
 __device__ __forceinline__ void ifft16(uint32_t rows, const In *in, uint4 *out, uint32_t b, uint32_t off,
                                        uint32_t limit) {
 #pragma unroll 1
   for (uint32_t lgd = 0; lgd < b; lgd += 2) {
     const bool last = lgd + 2 >= b;
-    pass16<NQ, false>(rows, lgd ? nullptr : in, last ? out : nullptr, 1u << b, lgd, lgd + 1 < b, off,
+    pass16<false>(rows, lgd ? nullptr : in, last ? out : nullptr, 1u << b, lgd, lgd + 1 < b, off,
                       last ? ~0u : limit, ~0u);
     __syncthreads();
   }
 }
 // FFT over 2^b rows into shared memory; the first pass reads `in`, unless null.
-template <int NQ>
 __device__ __forceinline__ void fft16(uint32_t rows, const ScratchRows *in, uint32_t b, uint32_t off, uint32_t limit,
                                       uint32_t need) {
   const uint32_t odd = b & 1;
 #pragma unroll 1
   for (int lgd = int(b) - 2 + int(odd); lgd >= 0; lgd -= 2) {
     const bool single = odd && lgd == int(b) - 1;
-    pass16<NQ, true>(rows, in, nullptr, 1u << b, uint32_t(lgd), !single, off, single ? ~0u : limit, single ? ~0u : need);
+    pass16<true>(rows, in, nullptr, 1u << b, uint32_t(lgd), !single, off, single ? ~0u : limit, single ? ~0u : need);
     in = nullptr;
     __syncthreads();
   }

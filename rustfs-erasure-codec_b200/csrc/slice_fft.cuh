@@ -460,7 +460,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
           if (info.ptr[r + j] & 1) {  // warp-uniform
             slice8(v[0]);
             planes_to_tower<8>(v[0]);
-            mac<8>(info.c[r + j], x, v[0]);
+            mac8(info.c[r + j], x, v[0]);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -513,7 +513,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
         const uint64_t ptr = info.ptr[r + j];
         if (ptr & 2) {  // warp-uniform
           uint32_t x[8] = {};
-          mac<8>(info.c[r + j], x, v[0]);
+          mac8(info.c[r + j], x, v[0]);
           planes_to_cantor<8>(x);
           slice8(x);
           cols.store(reinterpret_cast<uint8_t *>(ptr - 2), x);
@@ -537,7 +537,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
       cols.load(reinterpret_cast<const uint8_t *>(ptr - 1), y);
       slice8(y);
       planes_to_tower<8>(y);
-      mac<8>(info.c[i], x, y);
+      mac8(info.c[i], x, y);
     }
     s.store(s.at(i), x);
   }
@@ -556,7 +556,7 @@ __device__ __forceinline__ void slice_decode_tile(uint32_t smem, const SliceArgs
     if (!(ptr & 2)) continue;  // warp-uniform
     uint32_t y[8], x[8] = {};
     s.load(s.at(i), y);
-    mac<8>(info.c[i], x, y);
+    mac8(info.c[i], x, y);
     planes_to_cantor<8>(x);
     slice8(x);
     cols.store(reinterpret_cast<uint8_t *>(ptr - 2), x);

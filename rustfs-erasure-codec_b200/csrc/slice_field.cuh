@@ -225,16 +225,10 @@ __device__ __forceinline__ void sub2_nibble(uint32_t n, uint32_t *x0, const uint
                                             const uint32_t *y1);
 #include "slice_net.cuh"
 
-// x ^= c * y (one pair, two pairs) for a warp-uniform constant in tower
-// coordinates.
-template <int BITS>
-__device__ __forceinline__ void mac(uint32_t c, uint32_t *x, const uint32_t *y) {
-  mac_nibble<BITS, 0>(c & 15, x, y);
-  mac_nibble<BITS, 4>((c >> 4) & 15, x, y);
-  if (BITS == 16) {
-    mac_nibble<BITS, BITS == 16 ? 8 : 0>((c >> 8) & 15, x, y);
-    mac_nibble<BITS, BITS == 16 ? 12 : 0>((c >> 12) & 15, x, y);
-  }
+// x ^= c * y in GF(2^8) for a warp-uniform constant in tower coordinates.
+__device__ __forceinline__ void mac8(uint32_t c, uint32_t *x, const uint32_t *y) {
+  mac_nibble<8, 0>(c & 15, x, y);
+  mac_nibble<8, 4>((c >> 4) & 15, x, y);
 }
 // Tower coordinates of a Cantor constant, nibble by nibble.
 template <int BITS>
@@ -261,7 +255,7 @@ __device__ __forceinline__ uint32_t tower_const(uint32_t e) {
 // half the planes of GF(2^16) under its subfield GF(256).
 struct Gf8 {
   __device__ __forceinline__ static uint32_t tower(uint32_t e) { return tower_const<8>(e); }
-  __device__ __forceinline__ static void mac(uint32_t c, uint32_t *x, const uint32_t *y) { rsgpu::mac<8>(c, x, y); }
+  __device__ __forceinline__ static void mac(uint32_t c, uint32_t *x, const uint32_t *y) { mac8(c, x, y); }
   __device__ __forceinline__ static void mac2(uint32_t c, uint32_t *x0, const uint32_t *y0, uint32_t *x1,
                                               const uint32_t *y1) {
     mac2_nibble<8, 0>(c & 15, x0, y0, x1, y1);
