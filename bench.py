@@ -35,7 +35,7 @@ MIX_OPS = 16384  # stripes of the mixed-geometry workload
 # Both arms (this build and the reference's CPU path) report this metric.
 METRIC = "batched classic encode+rebuild+verify GB/s (algorithmic bytes)"
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
-PROFILE_FILE = os.path.join(ROOT, "profiles", "k_apply_tma_encode_10x4.txt")
+PROFILE_FILE = os.path.join(ROOT, "profiles", "k_apply_reg_encode_10x4.txt")
 
 
 def erasure_patterns(k, m, n, seed):

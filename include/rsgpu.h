@@ -357,9 +357,9 @@ typedef struct rsgpu_mix_op {
 
 /* Algorithms: RSGPU_ALGO_APPLY = the K1 table kernel over the operation's
  * coefficient matrix (classic; for Leopard GF(2^8) the FFT pipeline written
- * out as a dense matrix over the Leopard field); tile 0 = 8 KiB of columns and
- * four outputs per pass over the inputs, 1 = 4 KiB and four, 2 = 4 KiB and
- * eight.  RSGPU_ALGO_FFT = the Leopard transform, tile
+ * out as a dense matrix over the Leopard field), four outputs per pass over the
+ * inputs; tile 0 = 8 KiB of columns per work item, 1 = 4 KiB, 2 = as 1 (it was
+ * eight outputs per pass; plan tables that name it stay valid).  RSGPU_ALGO_FFT = the Leopard transform, tile
  * t = 2^t 64-byte column blocks per work item (t = 1..3; transforms of at
  * most 16 lanes run in registers on 1 KiB of columns whatever t is). */
 enum { RSGPU_ALGO_APPLY = 0, RSGPU_ALGO_FFT = 1 };
@@ -399,7 +399,8 @@ int32_t rsgpu_mix_launch(rsgpu_mix *mix, void *stream);
  * when the parity matched, 0 otherwise; other operations 1. */
 int32_t rsgpu_mix_results(rsgpu_mix *mix, uint8_t *ok, void *stream);
 int32_t rsgpu_mix_get_info(const rsgpu_mix *mix, rsgpu_mix_info *out);
-/* The plan chosen for each operation. */
+/* The plan chosen for each operation.  Leopard GF(2^8) operations that run in
+ * launches of their own (above) report the transform plan of the fixed rule. */
 int32_t rsgpu_mix_get_plans(const rsgpu_mix *mix, rsgpu_plan *out, size_t n_ops);
 void rsgpu_mix_free(rsgpu_mix *mix);
 

@@ -30,7 +30,7 @@
 //                     matrix: the classic matrix, or for Leopard GF(2^8) the
 //                     FFT pipeline written out as a dense matrix over the
 //                     Leopard field (exact: the pipeline is linear); tile 0 =
-//                     8 KiB of columns per item, 1 = 4 KiB;
+//                     8 KiB of columns per item, 1 and 2 = 4 KiB;
 //   RSGPU_ALGO_FFT    the Leopard transform tile, 2^tile 64-byte blocks per
 //                     item.
 // Every plan writes the same bytes; plans only change the speed.
@@ -74,8 +74,8 @@ constexpr int kMixThreads = 256;
 constexpr int kMixBlocks = 3;
 constexpr uint32_t kTailTile = 0xFFFFFFFFu;
 
-// K1 kinds: bits 0..1 = tile (0: 8 KiB of columns, 4 outputs per pass over
-// the inputs; 1: 4 KiB, 4; 2: 4 KiB, 8), bit 2 = verify.
+// K1 kinds: bits 0..1 = tile (0: 8 KiB of columns per item; 1, 2: 4 KiB), bit 2 =
+// verify.  2 was 8 outputs a pass; saved plans and the tuner's table still name it.
 enum MixKind : uint32_t {
   MK_APPLY = 0,
   MK_APPLY_VERIFY = 4,

@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(kApplyThreads + 32, 2) k_apply_tma(const __gri
 // the data read.  The staged tile above needs 8 shuffles and re-reads two
 // tables per input and step, in 96 registers; this one fits 72, so three CTAs
 // share an SM and the shuffle latency is hidden (10+4 encode, 1 MiB x 512:
-// 4498 -> 5351 GB/s while the clock is at its maximum, the pipe 81% busy; in
-// long runs under the power cap 4083 -> 4637, 72% of the copy peak).
+// 4498 -> 5351 GB/s while the clock is near its maximum, the pipe 81% busy; in
+// long runs deep in the power cap 4045 -> 4560, 71% of the copy peak).
 // A CTA takes a contiguous run of tiles: launches whose stripes carry
 // different tables then change tables once per stripe, not once per tile.
 // The producer warp, the mbarrier ring and its bounded waits are
