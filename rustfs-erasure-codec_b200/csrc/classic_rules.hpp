@@ -29,6 +29,18 @@ inline bool words_pay(bool verify, uint32_t max_out, uint64_t len, uint64_t n_jo
   return columns >= ((verify ? 256u : 704u) << 10) && 5 * columns >= 2 * padded;
 }
 
+// The same for launches that add to their outputs (n_in inputs: the changed
+// shards of an update).  The word kernel reads and writes each output word
+// between the others' bytes, so it needs inputs enough to pay for that: five, or
+// as many as there are outputs beyond four, and a few rounds of tiles.  One B200,
+// whole calls, bytes / words, us, shards of 4 MiB and of 16 MiB less 3 bytes:
+//   10+4 encode_single 43 / 70, 145 / 192;  update of 3: 65 / 80, 278 / 299,
+//   of 5: 78 / 88, 410 / 317, of 10: 145 / 109, 670 / 375
+//   50+20 of 10: 458 / 517, of 20: 724 / 679, of 50: 1751 / 1238 (1 MiB 474 / 425)
+inline bool words_pay_update(uint32_t n_in, uint32_t max_out, uint64_t len, uint64_t n_jobs) {
+  return n_in >= 5 && (max_out <= 4 || n_in >= max_out) && n_in * len * n_jobs >= (32u << 20);
+}
+
 // Whether a verify of n_in inputs a job runs in the staged tile rather than with
 // its tables in registers.  One or two inputs have next to no lookups to share,
 // and the register tile keeps fewer of their bytes on the way (every stage has

@@ -451,7 +451,9 @@ int ApplyLaunch::build(std::vector<JobDesc> &jobs, const std::vector<const uint8
   uint32_t max_out = 0, uni_in = jobs.empty() ? 0 : jobs[0].n_in;
   int any_vec = 0, any_unaligned = 0;
   for (const auto &j : jobs) max_out = std::max<uint32_t>(max_out, j.n_out);
-  const bool words = words_pay(vfy, max_out, len, jobs.size());  // how misaligned jobs go
+  // How misaligned jobs go.
+  const bool words = accumulate ? words_pay_update(jobs.empty() ? 0 : jobs[0].n_in, max_out, len, jobs.size())
+                                : words_pay(vfy, max_out, len, jobs.size());
   int tbl_stage = 0;
   for (auto &j : jobs) {
     tbl_stage |= j.tbl != jobs[0].tbl;

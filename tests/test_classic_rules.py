@@ -1,5 +1,5 @@
 """CPU: the rules that pick a kernel for misaligned classic shards and for
-verifies of few inputs (classic_rules.hpp) against times measured on one B200: on
+verifies of few inputs (classic_rules.hpp), updates among them, against times measured on one B200: on
 either side of their lines, the kernel they pick took at most 10% longer than the
 other."""
 import pathlib
@@ -54,6 +54,24 @@ FEW_INPUTS = [
     (STAGED, 4, 4096, 1024, 15, 20),
 ]
 
+UPDATE = 3
+# (, outputs + 1000 * inputs, shard length, stripes, us by bytes, us by words)
+UPDATES = [
+    (UPDATE, 1004, 4194301, 1, 43, 70),
+    (UPDATE, 1004, 16777213, 1, 145, 192),
+    (UPDATE, 3004, 16777213, 1, 278, 299),
+    (UPDATE, 5004, 4194301, 1, 78, 88),
+    (UPDATE, 5004, 16777213, 1, 410, 317),
+    (UPDATE, 10004, 1048573, 1, 43, 43),
+    (UPDATE, 10004, 4194301, 1, 145, 109),
+    (UPDATE, 5008, 4194301, 1, 120, 143),
+    (UPDATE, 10008, 4194301, 1, 234, 199),
+    (UPDATE, 10020, 4194301, 1, 458, 517),
+    (UPDATE, 20020, 4194301, 1, 724, 679),
+    (UPDATE, 50020, 1048573, 1, 474, 425),
+    (UPDATE, 50020, 4194301, 1, 1751, 1238),
+]
+
 _DRIVER = """
 #include <cstdio>
 #include "classic_rules.hpp"
@@ -61,7 +79,10 @@ int main() {
   unsigned verify, outs;
   unsigned long long len, stripes;
   while (scanf("%u %u %llu %llu", &verify, &outs, &len, &stripes) == 4)
-    puts((verify == 2 ? rsgpu::verify_staged(outs, len, stripes) : rsgpu::words_pay(verify, outs, len, stripes)) ? "1" : "0");
+    puts((verify == 3   ? rsgpu::words_pay_update(outs / 1000, outs % 1000, len, stripes)
+          : verify == 2 ? rsgpu::verify_staged(outs, len, stripes)
+                        : rsgpu::words_pay(verify, outs, len, stripes))
+             ? "1" : "0");
 }
 """
 
@@ -81,12 +102,12 @@ def _slow(cases, picks):
     return [c for c, second in zip(cases, picks) if c[5 if second else 4] > 1.1 * min(c[4:])]
 
 
-@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS])
+@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS, UPDATES])
 def test_rule_picks_the_faster_kernel(tmp_path, cases):
     assert not _slow(cases, _picks(tmp_path, cases))
 
 
-@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS])
+@pytest.mark.parametrize("cases", [TIMES, FEW_INPUTS, UPDATES])
 @pytest.mark.parametrize("second", [False, True])
 def test_a_wrong_rule_is_seen(cases, second):
     assert _slow(cases, [second] * len(cases))
